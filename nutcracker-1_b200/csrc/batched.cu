@@ -524,7 +524,7 @@ __global__ void lz_reduce_kernel(int nchains, const LzChain* __restrict__ ch, Lz
     if (c < nchains) reduce_chain<PASS>(c, lane, ch, st, part);
 }
 
-// One warp per chain: column j of the projected matrix from the
+// One block per chain: column j of the projected matrix from the
 // reorthogonalisation coefficients, the Ritz pairs (warm-started Jacobi,
 // nc_ritz.cuh), and the decision: converged (ARPACK's rule, Ritz estimate
 // <= tol * max(|theta|, eps^(2/3)), or the Krylov space exhausted or
@@ -537,9 +537,9 @@ __device__ __forceinline__ void ritz_chain(int c, RitzSmem<kMaxKrylov>& w, const
     const int j = S.j;
     LzRitz& R = rz[c];
     const RitzResult r =
-        ritz_update_warp<kMaxKrylov, false>(w, j + 1, R.state, S.h1, S.h2, fmax(S.wn2, 0.0), RITZ_SR, R.S,
-                                            kMaxKrylov, R.theta);
-    if ((threadIdx.x & 31) != 0) return;
+        ritz_update_block<kMaxKrylov, false>(w, j + 1, R.state, S.h1, S.h2, fmax(S.wn2, 0.0), RITZ_SR, R.S,
+                                             kMaxKrylov, R.theta);
+    if (threadIdx.x != 0) return;
     S.matvecs++;
     S.theta = r.theta;
     S.res = r.res;
@@ -557,9 +557,9 @@ __device__ __forceinline__ void ritz_chain(int c, RitzSmem<kMaxKrylov>& w, const
     }
 }
 
-__global__ void __launch_bounds__(32) lz_ritz_kernel(int nchains, const LzChain* __restrict__ ch,
-                                                     LzState* __restrict__ st, LzRitz* __restrict__ rz,
-                                                     int* __restrict__ active) {
+__global__ void __launch_bounds__(RITZ_THREADS) lz_ritz_kernel(int nchains, const LzChain* __restrict__ ch,
+                                                               LzState* __restrict__ st, LzRitz* __restrict__ rz,
+                                                               int* __restrict__ active) {
     __shared__ RitzSmem<kMaxKrylov> w;
     const int c = blockIdx.x;
     if (c == 0 && threadIdx.x == 0) *active = 0;
@@ -1776,7 +1776,7 @@ struct Engine {
         lz_reduce_kernel<1><<<cb, 256, 0, stream>>>(B, d_lz.p, st, d_part.p);
         lz_cgs_kernel<2><<<grid_vec, kLzT, 0, stream>>>(lz_chunks.d.p, lz_chunks.d_count.p, d_lz.p, st, d_part.p);
         lz_reduce_kernel<2><<<cb, 256, 0, stream>>>(B, d_lz.p, st, d_part.p);
-        lz_ritz_kernel<<<B, 32, 0, stream>>>(B, d_lz.p, st, d_rz.p, d_active.p);
+        lz_ritz_kernel<<<B, RITZ_THREADS, 0, stream>>>(B, d_lz.p, st, d_rz.p, d_active.p);
         lz_next_kernel<<<grid_vec, kLzT, 0, stream>>>(lz_chunks.d.p, lz_chunks.d_count.p, d_lz.p, st);
         // thick restart of the chains whose basis filled in this iteration
         lz_restart_form_kernel<<<grid_vec, kLzT, 0, stream>>>(lz_chunks.d.p, lz_chunks.d_count.p, d_lz.p, st, d_rz.p);

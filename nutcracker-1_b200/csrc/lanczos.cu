@@ -8,9 +8,8 @@
 // eigenpairs coincide).  Everything that touches vectors of length n runs on
 // the GPU: the H_eff product (contract.cu), the projector filter, the
 // reorthogonalisation (multi-dot / multi-axpy, HBM-bound) and the small
-// projected problem (Sturm multisection + inverse iteration for the
-// tridiagonal matrix, one warp).  The host only reads back three scalars per
-// step to decide convergence.
+// projected problem (warm-started Jacobi, one block, nc_ritz.cuh).  The host
+// only reads back three scalars per step to decide convergence.
 //
 // Convergence follows ARPACK's rule: the Ritz estimate beta_j |s_j| must be
 // <= tol * |theta| with tol >= machine epsilon.  `maxit` bounds the number of
@@ -255,14 +254,15 @@ __global__ void restart_t_kernel(int k, const double* __restrict__ theta, double
     ritz_restart_state<MAXT>(k, theta, state);
 }
 
-// Adds column m-1 of T to the kept decomposition and diagonalises (one warp);
+// Adds column m-1 of T to the kept decomposition and diagonalises (one block);
 // theta[] and S (m x m complex, column-major) receive the ordered Ritz pairs,
 // out the wanted pair's value and Ritz estimate.
-__global__ void ritz_kernel(int m, double* __restrict__ state, const cplx* __restrict__ h1,
-                            const cplx* __restrict__ h2, const cplx* __restrict__ nrm2, int which,
-                            RitzOut* __restrict__ out, cplx* __restrict__ S, double* __restrict__ theta) {
+__global__ void __launch_bounds__(RITZ_THREADS)
+ritz_kernel(int m, double* __restrict__ state, const cplx* __restrict__ h1, const cplx* __restrict__ h2,
+            const cplx* __restrict__ nrm2, int which, RitzOut* __restrict__ out, cplx* __restrict__ S,
+            double* __restrict__ theta) {
     __shared__ RitzSmem<MAXT> w;
-    const RitzResult r = ritz_update_warp<MAXT, true>(w, m, state, h1, h2, nrm2[0].x, which, S, m, theta);
+    const RitzResult r = ritz_update_block<MAXT, true>(w, m, state, h1, h2, nrm2[0].x, which, S, m, theta);
     if (threadIdx.x == 0) {
         out->theta = r.theta;
         out->res = r.res;
@@ -517,7 +517,7 @@ int optimize_site(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L
         filt.apply(ctx, n, w);
         ++st.matvecs;
         orthogonalise(w, j + 1);
-        ritz_kernel<<<1, 32, 0, ctx.stream>>>(j + 1, T, h1, h2, nr, which, ro, S, theta);
+        ritz_kernel<<<1, RITZ_THREADS, 0, ctx.stream>>>(j + 1, T, h1, h2, nr, which, ro, S, theta);
         NC_CHECK_LAUNCH();
         ctx.launches++;
         RitzOut rr;
