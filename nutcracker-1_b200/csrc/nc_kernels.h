@@ -174,6 +174,25 @@ void tc_check(Context& ctx);
 // leaves the first K stage of tile (0,0,0) unloaded (its wait then runs out).
 void tc_test_fault(unsigned long long wait_ns, int skip_first_load);
 
+// ---- complex128 GEMM through residues on the int8 tensor cores (residue_gemm.cu)
+// One operand: row i, K index k at X[(i % I) * si + (i / I) * sI + k * sk]
+// (sk == 1 or si == 1), conjugated when conj.
+struct ResMatrix {
+    const cplx* X = nullptr;
+    long long si = 0, sI = 0, sk = 0;
+    int I = 1, rows = 0, K = 0;
+    int conj = 0;
+};
+// Whether an M x N x K complex product is faster through residues than on the DMMA pipe.
+bool residue_gemm_pays(long long M, long long N, long long K);
+// C(m,n) = sum_k A(m,k) B(n,k) to C[(m % I) + (m / I) * sI + n * sn] (scratch
+// from ctx.scratch()).
+void residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b, cplx* C, int I, long long sI,
+                     long long sn);
+// Synchronises ctx.stream and raises NC_ERR_TIMEOUT if a wait of a residue
+// GEMM launched since the last check expired; returns at once when none was.
+void residue_check(Context& ctx);
+
 // ---- precision form of the site products (mixed.cu) ------------------------
 // Tensor-core operands of one site's H_eff (environments expanded once per
 // site) and the scratch of one product, all inside one float buffer of

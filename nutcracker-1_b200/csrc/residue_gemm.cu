@@ -1,0 +1,676 @@
+// Complex128 GEMM through residues on the int8 tensor cores (sm_100a).
+//
+// tcgen05 has no FP64 kind, and the FP64 tensor pipe (mma.sync DMMA,
+// zgemm.cu) gives 30 TFLOP/s; the int8 kind multiplies about a hundred times
+// faster.  So a large product C = A B runs in exact integer arithmetic modulo
+// L = 15 small coprime moduli (the "Ozaki scheme II" of Ozaki, Uchino and
+// Imamura 2025):
+//   1. every row of A and column of B is scaled by a power of two so that its
+//      2-norm lies in (2^57, 2^58], and rounded to integers;
+//   2. the integers' residues modulo each p_l fit in a byte (planes Re, Im and
+//      Re + Im, so that one complex product is three real ones);
+//   3. per modulus, three 8-bit GEMMs with int32 accumulation in tensor memory
+//      give P1 = Re Re, P2 = Im Im, P3 = (Re + Im)(Re + Im); the epilogue
+//      reduces Re C = P1 - P2 and Im C = P3 - P1 - P2 modulo p_l to a byte;
+//   4. the Chinese remainder theorem rebuilds each integer of C from its L
+//      residues, and the scales are undone.
+// By Cauchy-Schwarz |C_mn| <= 2^116 before the scales are undone, and the
+// product of the moduli is above 2^117.8, so steps 2 to 4 are exact: the only
+// error is the rounding in step 1, 2^-59 of a row's norm per element, and one
+// final rounding.  Measured against exact values, the error is below the
+// DMMA kernel's, whose accumulation rounds at every term (see
+// residue_gemm_pays for the figures and for where this route begins).
+//
+// Kernels: norms (HBM read), residues (HBM: 16 bytes read, 45 written per
+// complex element), the GEMM (tensor-bound), CRT (HBM: 30 bytes read, 16
+// written per element).  The GEMM is one persistent CTA per SM over
+// (modulus, column tile, row tile) items: a 128 x 256 tile of one plane's
+// product at a time (tcgen05.mma.kind::i8, 128 x 256 x 32 per instruction),
+// 128-byte K stages through a 4-deep TMA ring, two 256-column accumulators
+// in tensor memory that alternate between planes so that the epilogue of one
+// overlaps the MMAs of the next.  A non-finite row or column gives NaN.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <string>
+
+#include "nc_common.cuh"
+#include "nc_kernels.h"
+#include "nc_tcgen05.cuh"
+
+namespace nc {
+
+namespace {
+
+// ---- moduli and the constants of the Chinese remainder theorem --------------
+constexpr int NL = 15;
+constexpr int kMod[NL] = {256, 253, 251, 247, 245, 243, 241, 239, 233, 229, 227, 223, 211, 199, 197};
+constexpr int kNormBits = 58;         // scaled rows: 2-norm in (2^57, 2^58]
+constexpr int kSplit = 77;            // CRT weights split at 2^77
+typedef unsigned __int128 u128;
+
+constexpr u128 mod_product() {
+    u128 p = 1;
+    for (int l = 0; l < NL; ++l) p *= (u128)kMod[l];
+    return p;
+}
+// (P / p_l) * ((P / p_l)^-1 mod p_l): 1 modulo p_l, 0 modulo the others
+constexpr u128 crt_weight(int l) {
+    const u128 q = mod_product() / (u128)kMod[l];
+    const int r = (int)(q % (u128)kMod[l]);
+    int inv = 1;
+    while ((inv * r) % kMod[l] != 1) ++inv;
+    return q * (u128)inv;
+}
+constexpr double hi_part(u128 x) { return (double)(unsigned long long)(x >> kSplit); }
+constexpr double lo_part(u128 x) {
+    const u128 y = x & (((u128)1 << kSplit) - 1);
+    return (double)(unsigned long long)(y >> 20) * 1048576.0 + (double)(unsigned long long)(y & 1048575);
+}
+constexpr int pow2_mod(int e, int p) {
+    int r = 1;
+    for (int i = 0; i < e; ++i) r = (2 * r) % p;
+    return r;
+}
+static_assert((mod_product() >> 117) == 1, "2 * 2^(2 kNormBits) < P < 2^118");
+
+constexpr float kMagicF = 12582912.0f;      // 1.5 * 2^23: a float added to it is rounded to an integer
+constexpr unsigned kMagicI = 0x4B400000u;   // its bits: kMagicI + i is the float kMagicF + i, |i| < 2^22
+constexpr int kBias = 59;   // integers are stored plus 2^59: 0 < v < 2^60
+struct Tables {
+    unsigned p[NL];               // modulus
+    float invf[NL], half[NL];     // 1 / p, kMagicF + floor(p / 2)
+    unsigned m0[NL], m1[NL];      // 2^(8 i) modulo p for the low and the high four bytes, packed
+    unsigned off[NL];             // kMagicI + (minus 2^kBias modulo p)
+    int inv38[NL];                // 2^38 / p, rounded
+    double wh[NL], wl[NL];        // CRT weights: wh * 2^77 + wl
+};
+constexpr Tables make_tables() {
+    Tables t{};
+    for (int l = 0; l < NL; ++l) {
+        const int p = kMod[l];
+        t.p[l] = (unsigned)p;
+        t.invf[l] = 1.0f / (float)p;
+        t.half[l] = kMagicF + (float)(p / 2);
+        for (int i = 0; i < 4; ++i) {
+            t.m0[l] |= (unsigned)pow2_mod(8 * i, p) << (8 * i);
+            t.m1[l] |= (unsigned)pow2_mod(32 + 8 * i, p) << (8 * i);
+        }
+        t.off[l] = kMagicI + (unsigned)((p - pow2_mod(kBias, p)) % p);
+        t.inv38[l] = (int)(((1ull << 38) + p / 2) / p);
+        t.wh[l] = hi_part(crt_weight(l));
+        t.wl[l] = lo_part(crt_weight(l));
+    }
+    return t;
+}
+__constant__ Tables kT = make_tables();
+constexpr double kPh = hi_part(mod_product()), kPl = lo_part(mod_product());
+constexpr int kBadExp = 1 << 30;         // exponent of a row with a non-finite element
+constexpr int kMaxK = 16000;             // |Re|, |Im| sums of K residue products fit in int32
+
+__device__ int g_res_error = 0;
+constexpr unsigned long long kWaitNs = 2000000000ull;
+
+// four values' low bytes
+__device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
+
+// ---- operands ------------------------------------------------------------------
+// Row i, K index k of a complex operand: X[(i % I) * si + (i / I) * sI + k * sk].
+struct ResSource {
+    const cplx* X;
+    long long si, sI, sk;
+    int I, rows, K;
+    int conj;
+};
+
+constexpr int NT = 256;
+
+__device__ __forceinline__ const cplx* row_ptr(const ResSource& s, int i) {
+    return s.X + (long long)(i % s.I) * s.si + (long long)(i / s.I) * s.sI;
+}
+
+// One launch handles both operands of a product (the first nb[0] blocks along
+// x are operand 0's), so that a small product does not wait for two launches.
+struct ResPair {
+    ResSource s[2];
+    double2* part[2];     // [K chunk][row]
+    int* exps[2];
+    uint8_t* planes[2];
+    int nb[2], nchunk[2], chunk[2];
+    int Kp, lper;         // padded K; moduli per block
+};
+
+// Per (K chunk, row): sum |x|^2 and max(|Re|, |Im|).  K contiguous: one block
+// per row and chunk; else 32 rows per block, lanes along the rows.
+__global__ void __launch_bounds__(NT) res_norm_kernel(ResPair P) {
+    __shared__ double2 red[NT];
+    const int w2 = (int)blockIdx.x >= P.nb[0] ? 1 : 0, bx = blockIdx.x - (w2 ? P.nb[0] : 0);
+    const ResSource& s = P.s[w2];
+    if ((int)blockIdx.y >= P.nchunk[w2]) return;
+    double2* part = P.part[w2];
+    const int k0 = blockIdx.y * P.chunk[w2], k1 = min(s.K, k0 + P.chunk[w2]);
+    double sum = 0, mx = 0;
+    auto take = [&](const cplx v) {
+        sum = fma(v.x, v.x, fma(v.y, v.y, sum));     // a NaN survives here, fmax drops it
+        mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
+    };
+    if (s.sk == 1) {
+        const cplx* x = row_ptr(s, bx);
+        for (int k = k0 + threadIdx.x; k < k1; k += NT) take(x[k]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        }
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_double2(sum, mx);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int q = 1; q < NT / 32; ++q) {
+                sum += red[q].x;
+                mx = fmax(mx, red[q].y);
+            }
+            part[(size_t)blockIdx.y * s.rows + bx] = make_double2(sum, mx);
+        }
+    } else {
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        const int row = bx * 32 + lane;
+        if (row < s.rows) {
+            const cplx* x = row_ptr(s, row);
+#pragma unroll 4
+            for (int k = k0 + w; k < k1; k += NT / 32) take(x[(long long)k * s.sk]);
+        }
+        red[threadIdx.x] = make_double2(sum, mx);
+        __syncthreads();
+        if (w == 0 && row < s.rows) {
+            for (int q = 1; q < NT / 32; ++q) {
+                sum += red[q * 32 + lane].x;
+                mx = fmax(mx, red[q * 32 + lane].y);
+            }
+            part[(size_t)blockIdx.y * s.rows + row] = make_double2(sum, mx);
+        }
+    }
+}
+
+// Scale exponent e of each row (the row times 2^e has its 2-norm in
+// (2^57, 2^58]), or kBadExp when an element is not finite.
+__device__ __forceinline__ int row_exponent(const double2* __restrict__ part, int nchunk, int rows, int row, int K) {
+    double sum = 0, mx = 0;
+    for (int c = 0; c < nchunk; ++c) {
+        const double2 v = part[(size_t)c * rows + row];
+        sum += v.x;
+        mx = fmax(mx, v.y);
+    }
+    if (isnan(sum) || isinf(mx)) return kBadExp;
+    if (mx == 0.0) return 0;
+    int e = 0;
+    if (sum > 1e-270 && sum < 1e270) {
+        frexp(sqrt(sum) * (1.0 + 1e-12), &e);                 // norm <= 2^e
+    } else {                                                  // squares out of range: bound by the largest element
+        frexp(mx, &e);
+        int b = 0;
+        frexp(sqrt(2.0 * K), &b);
+        e += b;
+    }
+    return min(kNormBits - e, 1000);
+}
+
+// Residues of 16 rows x 128 K of an operand: planes[(3 l + c)][row][Kp] bytes,
+// c = Re, Im, Re + Im.  Bound by instruction issue: 23 million complex
+// elements (the operands of a chi=1024 Heisenberg product) write 1 GB, 0.16 ms
+// at the HBM rate, and cost 15 x 13 integer instructions each.  A residue of
+// the 60-bit integer is two dot products of its bytes with the powers of 2^8
+// modulo p (dp4a), one high multiplication by 2^32 / p and one multiply-add.
+// A thread makes four consecutive K of a row at a time, so that a warp writes
+// a whole 128-byte line of each plane.  A grid too small for the chip is split
+// over the moduli as well.
+constexpr int CR = 16, CK = 128;
+// kMagicI (1 - p) + the residue, which is in [0, p): t = 2^8 powers modulo p
+// times the bytes, as the bits of a float; q = round((t - p/2) / p).
+__device__ __forceinline__ uint32_t residue(uint2 v, uint32_t m0, uint32_t m1, uint32_t off, float inv, float half,
+                                            uint32_t p) {
+    const uint32_t t = __dp4a(v.y, m1, __dp4a(v.x, m0, off));   // kMagicI + t, t < 2^20
+    const float q = fmaf(__uint_as_float(t) - half, inv, kMagicF);
+    return t - __float_as_uint(q) * p;
+}
+__device__ __forceinline__ uint2 biased(double x, double scale) {
+    const unsigned long long v = (unsigned long long)(__double2ll_rn(x * scale) + (1ll << kBias));
+    return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+}
+__global__ void __launch_bounds__(NT, 4) res_convert_kernel(ResPair P) {
+    __shared__ cplx tile[CR][CK + 1];
+    __shared__ double scale[CR];
+    const int w2 = (int)blockIdx.x >= P.nb[0] ? 1 : 0, bx = blockIdx.x - (w2 ? P.nb[0] : 0);
+    const ResSource& s = P.s[w2];
+    const int kb = (P.Kp + CK - 1) / CK;
+    const int r0 = (bx / kb) * CR, k0 = (bx % kb) * CK;
+    const int tid = threadIdx.x;
+    if (tid < CR) {
+        const int row = r0 + tid;
+        int e = 0;
+        if (row < s.rows) {
+            e = row_exponent(P.part[w2], P.nchunk[w2], s.rows, row, s.K);
+            if (k0 == 0 && blockIdx.y == 0) P.exps[w2][row] = e;
+        }
+        scale[tid] = (e == kBadExp) ? 0.0 : scalbn(1.0, e);
+    }
+    for (int e = tid; e < CR * CK; e += NT) {
+        const int r = (s.sk == 1) ? e / CK : e % CR, k = (s.sk == 1) ? e % CK : e / CR;
+        const int row = r0 + r, kk = k0 + k;
+        tile[r][k] = (row < s.rows && kk < s.K) ? row_ptr(s, row)[(long long)kk * s.sk] : cmake(0, 0);
+    }
+    __syncthreads();
+    const size_t plane = (size_t)s.rows * P.Kp;
+    const int l0 = blockIdx.y * P.lper, l1 = min(NL, l0 + P.lper), k = (tid & 31) * 4;
+    for (int r = tid >> 5; r < CR; r += NT / 32) {
+        const int row = r0 + r;
+        if (row >= s.rows || k0 + k >= P.Kp) break;
+        const double sc = scale[r];
+        uint2 vr[4], vi[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            cplx v = tile[r][k + q];
+            if (sc == 0.0) v = cmake(0, 0);
+            vr[q] = biased(v.x, sc);
+            vi[q] = biased(s.conj ? -v.y : v.y, sc);
+        }
+        uint8_t* out = P.planes[w2] + (size_t)row * P.Kp + k0 + k + (size_t)(3 * l0) * plane;
+#pragma unroll 3
+        for (int l = l0; l < l1; ++l, out += 3 * plane) {
+            const uint32_t p = kT.p[l], m0 = kT.m0[l], m1 = kT.m1[l], off = kT.off[l];
+            const float inv = kT.invf[l], half = kT.half[l];
+            const uint32_t twice = 2 * (kMagicI * (p - 1));
+            uint32_t a[4], b[4], c[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                a[q] = residue(vr[q], m0, m1, off, inv, half, p);
+                b[q] = residue(vi[q], m0, m1, off, inv, half, p);
+                const uint32_t sum = a[q] + b[q] + twice;
+                c[q] = min(sum, sum - p);   // the wrapped difference is large when sum < p
+            }
+            *reinterpret_cast<uint32_t*>(out) = pack4(a[0], a[1], a[2], a[3]);
+            *reinterpret_cast<uint32_t*>(out + plane) = pack4(b[0], b[1], b[2], b[3]);
+            *reinterpret_cast<uint32_t*>(out + 2 * plane) = pack4(c[0], c[1], c[2], c[3]);
+        }
+    }
+}
+
+// ---- the GEMM ----------------------------------------------------------------------
+constexpr int TM = 128, TN = 256, TKB = 128;   // tile rows, columns, K bytes per stage
+constexpr int STAGES = 4;
+constexpr int A_STAGE = TM * TKB, B_STAGE = TN * TKB;
+constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
+constexpr int EPI_WARPS = 16, EPI_FIRST = 2;   // warps 0, 1: loads, MMAs
+constexpr int EPI_COLS = 4 * TN / EPI_WARPS;   // columns per epilogue warp
+constexpr int RG_THREADS = 32 * (EPI_FIRST + EPI_WARPS);
+constexpr int TMEM_COLS = 512;
+constexpr int CHUNK = 8;                        // columns per tensor-memory load
+constexpr size_t RG_SMEM = (size_t)STAGES * STAGE_BYTES + 1024 + 256;
+
+// kind::i8: D s32, A and B u8, both K-major, M x N.
+constexpr uint32_t IDESC_I8 = (2u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+
+__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+        "l"(da), "l"(db), "r"(IDESC_I8), "r"(accumulate)
+        : "memory");
+}
+
+struct ResGemm {
+    int M, N, nkb, mt, nt;   // K stages, row and column tiles
+    int n4, mp;              // column groups of four and rows, padded to whole tiles
+    uint32_t* res;           // [l][Re, Im][n4][mp] words of four columns
+};
+
+// v modulo p in [0, p] (p itself for some multiples of p), |v| < 2^31: the
+// quotient's error |v| / 2^39 stays below 1 / 256, so that flooring it is
+// wrong at multiples of p only.
+__device__ __forceinline__ uint32_t mod_int(int v, int p, int inv38) {
+    return (uint32_t)(v - (__mulhi(v, inv38) >> 6) * p);
+}
+
+__device__ __forceinline__ void tmem_ldc(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(RG_THREADS, 1)
+residue_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, ResGemm P) {
+    extern __shared__ unsigned char rg_smem_raw[];
+    const uint32_t raw = su32(rg_smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    const uint32_t bars = base + STAGES * STAGE_BYTES;
+    const uint32_t full0 = bars, empty0 = bars + 8 * STAGES;
+    const uint32_t accf0 = bars + 16 * STAGES, acce0 = accf0 + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rg_smem_raw + (acce0 + 16 - raw));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(full0 + 8 * s, 1);
+            mbar_init(empty0 + 8 * s, 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(accf0 + 8 * b, 1);
+            mbar_init(acce0 + 8 * b, EPI_WARPS);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tmem_slot)),
+                     "r"(TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_d = *tmem_slot;
+    const int tiles = P.mt * P.nt, items = tiles * NL;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int t = 0;
+            bool ok = true;
+            for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+                const int l = it / tiles, q = it % tiles, m0 = (q % P.mt) * TM, n0 = (q / P.mt) * TN;
+                for (int c = 0; c < 3 && ok; ++c)
+                    for (int kb = 0; kb < P.nkb; ++kb, ++t) {
+                        const int s = t % STAGES;
+                        if (!mbar_wait(empty0 + 8 * s, ((uint32_t)(t / STAGES) & 1u) ^ 1u, kWaitNs, &g_res_error)) {
+                            ok = false;
+                            break;
+                        }
+                        mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
+                        tma_load_3d(base + s * STAGE_BYTES, &mapA, kb * TKB, m0, 3 * l + c, full0 + 8 * s);
+                        tma_load_3d(base + s * STAGE_BYTES + A_STAGE, &mapB, kb * TKB, n0, 3 * l + c, full0 + 8 * s);
+                    }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            int t = 0, pass = 0;
+            bool ok = true;
+            for (int it = blockIdx.x; it < items && ok; it += gridDim.x)
+                for (int c = 0; c < 3 && ok; ++c, ++pass) {
+                    const int b = pass & 1;
+                    const uint32_t acc = tmem_d + (uint32_t)(b * TN);
+                    if (!mbar_wait(acce0 + 8 * b, ((uint32_t)(pass >> 1) & 1u) ^ 1u, kWaitNs, &g_res_error)) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    for (int kb = 0; kb < P.nkb; ++kb, ++t) {
+                        const int s = t % STAGES;
+                        if (!mbar_wait(full0 + 8 * s, (uint32_t)(t / STAGES) & 1u, kWaitNs, &g_res_error)) {
+                            ok = false;
+                            break;
+                        }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint64_t da = smem_desc(base + s * STAGE_BYTES);
+                        const uint64_t db = smem_desc(base + s * STAGE_BYTES + A_STAGE);
+#pragma unroll
+                        for (int ks = 0; ks < TKB / 32; ++ks)   // 32 bytes of K per instruction
+                            mma_i8(acc, da + 2 * ks, db + 2 * ks, (kb | ks) ? 1u : 0u);
+                        mma_commit(empty0 + 8 * s);
+                    }
+                    mma_commit(accf0 + 8 * b);
+                }
+        }
+    } else if (warp >= EPI_FIRST) {
+        // epilogue: warp w drains TMEM lanes 32*(w%4) .. +31 (a warp can reach
+        // only those), columns [EPI_COLS h, EPI_COLS (h + 1)), h = (w-2)/4
+        const int q = warp & 3, h = (warp - EPI_FIRST) >> 2;
+        int pass = 0;
+        bool ok = true;
+        for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+            const int l = it / tiles, tq = it % tiles;
+            const int m = (tq % P.mt) * TM + q * 32 + lane, n0 = (tq / P.mt) * TN + h * EPI_COLS;
+            const int p = (int)kT.p[l], inv = kT.inv38[l];
+            int acc[EPI_COLS];   // P1, then P1 + P2
+#pragma unroll 1
+            for (int c = 0; c < 3; ++c, ++pass) {
+                const int b = pass & 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (uint32_t)(pass >> 1) & 1u, kWaitNs, &g_res_error));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t src = tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * TN + h * EPI_COLS);
+                if (c == 0) {
+#pragma unroll
+                    for (int i = 0; i < EPI_COLS / CHUNK; ++i) {
+                        uint32_t v[CHUNK];
+                        tmem_ldc(src + CHUNK * i, v);
+#pragma unroll
+                        for (int e = 0; e < CHUNK; ++e) acc[CHUNK * i + e] = (int)v[e];
+                    }
+                } else {
+                    // whole tiles are stored: res is padded to them
+                    uint32_t* out = P.res + ((size_t)(2 * l + (c >> 1)) * P.n4 + n0 / 4) * P.mp + m;
+                    const int sx = c == 1 ? -1 : 1;   // c = 1: P1 - P2; c = 2: P3 - (P1 + P2)
+#pragma unroll
+                    for (int i = 0; i < EPI_COLS / CHUNK; ++i) {
+                        uint32_t v[CHUNK];
+                        tmem_ldc(src + CHUNK * i, v);
+#pragma unroll
+                        for (int e = 0; e < CHUNK; e += 4) {
+                            uint32_t r[4];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const int x = (int)v[e + u], y = acc[CHUNK * i + e + u];
+                                r[u] = mod_int(sx * (x - y), p, inv);
+                                acc[CHUNK * i + e + u] = y + x;
+                            }
+                            *out = pack4(r[0], r[1], r[2], r[3]);
+                            out += P.mp;
+                        }
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acce0 + 8 * b) : "memory");
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(TMEM_COLS)
+                     : "memory");
+    }
+}
+
+// ---- Chinese remainder theorem ---------------------------------------------------------
+struct ResOut {
+    cplx* C;
+    int M, N, n4, mp, I;          // row m = (m % I) * 1 + (m / I) * sI
+    long long sI, sn;
+    const int *ea, *eb;       // scale exponents of A's rows and B's columns
+};
+
+// S = sum_l r_l W_l as S_h 2^77 + S_l (S_h exact: 15 * 255 * 2^41 < 2^53), the
+// multiple of P removed: the integer of C, rounded once to FP64.
+__device__ __forceinline__ double crt(const uint32_t (&w)[NL], int byte) {
+    double sh = 0, sl = 0;
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+        const double d = __hiloint2double(0x43300000, __byte_perm(w[l], 0, 0x4440 | byte)) - 4503599627370496.0;
+        sh = fma(d, kT.wh[l], sh);
+        sl = fma(d, kT.wl[l], sl);
+    }
+    const double k = rint(sh * (1.0 / kPh));
+    sh = fma(-k, kPh, sh);
+    sl = fma(-k, kPl, sl);
+    return fma(sh, 151115727451828646838272.0, sl);   // 2^77
+}
+
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+
+__global__ void __launch_bounds__(128) res_crt_kernel(const uint32_t* __restrict__ res, ResOut o) {
+    const int m = blockIdx.x * 128 + threadIdx.x, g = blockIdx.y;
+    if (m >= o.M) return;
+    uint32_t wr[NL], wi[NL];
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+        wr[l] = res[((size_t)(2 * l) * o.n4 + g) * o.mp + m];
+        wi[l] = res[((size_t)(2 * l + 1) * o.n4 + g) * o.mp + m];
+    }
+    const int ea = o.ea[m];
+    cplx* row = o.C + (m % o.I) + (long long)(m / o.I) * o.sI;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int n = 4 * g + u;
+        if (n >= o.N) break;
+        const int eb = o.eb[n];
+        cplx v;
+        if (ea == kBadExp || eb == kBadExp) {
+            const double nan = __longlong_as_double(0x7ff8000000000000ll);
+            v = cmake(nan, nan);
+        } else {
+            // undo 2^(ea + eb) in three factors, so that no factor leaves FP64's range
+            const int e = -(ea + eb), e1 = e / 3, e2 = (e - e1) / 2;
+            const double f1 = pow2(e1), f2 = pow2(e2), f3 = pow2(e - e1 - e2);
+            v = cmake(crt(wr, u) * f1 * f2 * f3, crt(wi, u) * f1 * f2 * f3);
+        }
+        row[(long long)n * o.sn] = v;
+    }
+}
+
+// rows x Kp int8, 3 NL planes
+CUtensorMap make_map8(const uint8_t* ptr, int Kp, int rows, int rows_p, int box_rows) {
+    CUtensorMap m;
+    std::memset(&m, 0, sizeof(m));
+    const cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)rows, (cuuint64_t)(3 * NL)};
+    const cuuint64_t strides[2] = {(cuuint64_t)Kp, (cuuint64_t)Kp * rows_p};
+    const cuuint32_t box[3] = {(cuuint32_t)TKB, (cuuint32_t)box_rows, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(ptr), dims, strides, box, estr,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+        throw Error(NC_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
+    return m;
+}
+
+}  // namespace
+
+// Measured on a B200, one H_eff product of a Heisenberg site (two GEMMs and
+// the mix), DMMA route against this one: chi = 192 80 / 116 us, 224 109 / 129,
+// 256 200 / 142, 320 352 / 182, 512 1020 / 369, 1024 5750 / 1440.  The
+// crossing lies near 2^27 complex multiplications a GEMM; below one tile of
+// rows or half a tile of columns the padding costs more.  Error against
+// extended precision (2-norm, chi = 256 / 1024): DMMA 4.3e-16 / 2.2e-15, this
+// route 1.4e-16 / 2.9e-16.  The error is relative to the norms of the rows of
+// A and the columns of B: an output far below |a_m| |b_n| can be off by more
+// than its own rounding.
+bool residue_gemm_pays(long long M, long long N, long long K) {
+    return M >= TM && N >= TN / 2 && K >= 64 && K <= kMaxK && M * N * K >= (1LL << 27);
+}
+
+namespace {
+struct ResOperand {
+    uint8_t* planes;
+    int* exps;
+    int rows, K, Kp;
+};
+
+int padded_k(int K) { return (K + 63) / 64 * 64; }
+
+// Residue planes and row scales of both operands (scratch of the caller's frame).
+void residue_convert(Context& ctx, const ResMatrix* const (&src)[2], ResOperand (&out)[2]) {
+    Arena& ar = ctx.scratch();
+    ResPair P;
+    P.Kp = padded_k(src[0]->K);
+    int ny = 1;
+    for (int w = 0; w < 2; ++w) {
+        const ResMatrix& a = *src[w];
+        NC_ARG(a.rows >= 1 && a.K >= 1 && a.I >= 1 && (a.sk == 1 || a.si == 1), "residue operand: bad layout");
+        ResSource& s = P.s[w];
+        s.X = a.X; s.si = a.si; s.sI = a.sI; s.sk = a.sk; s.I = a.I; s.rows = a.rows; s.K = a.K; s.conj = a.conj;
+        P.planes[w] = ar.alloc_n<uint8_t>((size_t)3 * NL * a.rows * P.Kp);
+        P.exps[w] = ar.alloc_n<int>(a.rows);
+        out[w] = ResOperand{P.planes[w], P.exps[w], a.rows, a.K, P.Kp};
+        // enough blocks for the chip: long K in chunks
+        P.nb[w] = (a.sk == 1) ? a.rows : (a.rows + 31) / 32;
+        const int want = std::max(1, std::min((4 * 148 + P.nb[w] - 1) / P.nb[w], (a.K + 63) / 64));
+        P.chunk[w] = (a.K + want - 1) / want;
+        P.nchunk[w] = (a.K + P.chunk[w] - 1) / P.chunk[w];
+        P.part[w] = ar.alloc_n<double2>((size_t)P.nchunk[w] * a.rows);
+        ny = std::max(ny, P.nchunk[w]);
+    }
+    res_norm_kernel<<<dim3(P.nb[0] + P.nb[1], ny), NT, 0, ctx.stream>>>(P);
+    NC_CHECK_LAUNCH();
+    long long blocks = 0;
+    for (int w = 0; w < 2; ++w) {
+        const long long nb = (long long)((P.Kp + CK - 1) / CK) * ((P.s[w].rows + CR - 1) / CR);
+        P.nb[w] = (int)nb;
+        blocks += nb;
+    }
+    NC_ARG(blocks < (1LL << 31), "residue operand: too large");
+    P.lper = blocks < 2 * 148 ? 3 : blocks < 4 * 148 ? 5 : NL;
+    res_convert_kernel<<<dim3((unsigned)blocks, (NL + P.lper - 1) / P.lper), NT, 0, ctx.stream>>>(P);
+    NC_CHECK_LAUNCH();
+    ctx.launches += 2;
+}
+
+void residue_gemm(Context& ctx, const ResOperand& A, const ResOperand& B, cplx* C, int I, long long sI, long long sn) {
+    NC_ARG(A.K == B.K && A.K <= kMaxK, "residue GEMM: K");
+    NC_SET_SMEM_ONCE(residue_gemm_kernel, RG_SMEM);
+    ArenaFrame f(ctx.scratch());
+    ResGemm P;
+    P.M = A.rows; P.N = B.rows;
+    P.nkb = (A.Kp + TKB - 1) / TKB;
+    P.mt = (P.M + TM - 1) / TM; P.nt = (P.N + TN - 1) / TN;
+    P.n4 = P.nt * (TN / 4);
+    P.mp = P.mt * TM;
+    P.res = ctx.scratch().alloc_n<uint32_t>((size_t)2 * NL * P.n4 * P.mp);
+    const CUtensorMap ma = make_map8(A.planes, A.Kp, A.rows, A.rows, TM);
+    const CUtensorMap mb = make_map8(B.planes, B.Kp, B.rows, B.rows, TN);
+    const long long items = (long long)P.mt * P.nt * NL;
+    NC_ARG(items < (1LL << 31), "residue GEMM: too large");
+    residue_gemm_kernel<<<(unsigned)std::min<long long>(items, 148), RG_THREADS, RG_SMEM, ctx.stream>>>(ma, mb, P);
+    NC_CHECK_LAUNCH();
+    ResOut o;
+    o.C = C; o.M = P.M; o.N = P.N; o.n4 = P.n4; o.mp = P.mp; o.I = I; o.sI = sI; o.sn = sn; o.ea = A.exps; o.eb = B.exps;
+    const int groups = (P.N + 3) / 4;
+    NC_ARG(groups <= 65535, "residue GEMM: too many columns");
+    res_crt_kernel<<<dim3((P.M + 127) / 128, groups), 128, 0, ctx.stream>>>(P.res, o);
+    NC_CHECK_LAUNCH();
+    ctx.launches += 2;
+    ctx.residue_used = true;
+}
+
+}  // namespace
+
+void residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b, cplx* C, int I, long long sI,
+                     long long sn) {
+    NC_ARG(a.K == b.K, "residue product: K");
+    profile_launch(ctx, 8.0 * a.rows * (double)b.rows * a.K, 0, [&] {
+        ArenaFrame f(ctx.scratch());
+        const ResMatrix* const src[2] = {&a, &b};
+        ResOperand op[2];
+        residue_convert(ctx, src, op);
+        residue_gemm(ctx, op[0], op[1], C, I, sI, sn);
+    });
+}
+
+void residue_check(Context& ctx) {
+    if (!ctx.residue_used) return;
+    ctx.residue_used = false;
+    NC_CUDA(cudaStreamSynchronize(ctx.stream));
+    int flag = 0;
+    NC_CUDA(cudaMemcpyFromSymbol(&flag, g_res_error, sizeof(int)));
+    if (flag) {
+        const int zero = 0;
+        NC_CUDA(cudaMemcpyToSymbol(g_res_error, &zero, sizeof(int)));
+        throw Error(NC_ERR_TIMEOUT, "residue GEMM: a pipeline wait exceeded its time limit");
+    }
+}
+
+}  // namespace nc

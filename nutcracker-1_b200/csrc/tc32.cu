@@ -27,13 +27,12 @@
 // thread.  The epilogue stores complex64 or complex128 to any strided
 // layout.  No multicast; every mbarrier wait is bounded by the global timer
 // and reports through g_tc_error.
-#include <cuda.h>
-
 #include <cstring>
 #include <string>
 
 #include "nc_common.cuh"
 #include "nc_kernels.h"
+#include "nc_tcgen05.cuh"
 
 namespace nc {
 
@@ -72,61 +71,6 @@ struct TcParams {
     int c_fp64;
 };
 
-__device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ unsigned long long gtimer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// Bounded wait: false (and g_tc_error set) when the phase did not complete in `limit` ns.
-__device__ __noinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned long long limit) {
-    if (mbar_test(bar, parity)) return true;
-    const unsigned long long t0 = gtimer();
-    while (!mbar_test(bar, parity)) {
-        if (gtimer() - t0 > limit) {
-            atomicExch(&g_tc_error, 1);
-            return false;
-        }
-    }
-    return true;
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
-                                            uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-        : "memory");
-}
-
-// K-major operand tile in the 128-byte-swizzled layout written by TMA:
-// 8-row x 128-byte atoms, 1024 bytes apart (SBO); LBO unused for this layout.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-
 // kind::tf32 instruction descriptor: D f32, A/B tf32, both K-major, M x N.
 constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TN >> 3) << 17) |
                            ((uint32_t)(TM >> 4) << 24);
@@ -137,24 +81,6 @@ __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t da, uint64_t 
         " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
         "l"(da), "l"(db), "r"(IDESC), "r"(accumulate)
         : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-        "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
-          "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
-          "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 __global__ void __launch_bounds__(TC_THREADS, 1)
@@ -211,7 +137,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
                     for (int kb = kb0; kb < kb1; ++kb, ++t) {
                         const int s = t % STAGES;
                         const uint32_t ph = (uint32_t)(t / STAGES) & 1u;
-                        if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, limit)) { ok = false; break; }
+                        if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, limit, &g_tc_error)) { ok = false; break; }
                         if (skip_first && t == 0) continue;   // test switch: stage 0 never arrives
                         const CUtensorMap* ma = (seg == 2) ? &mapAs : &mapAb;
                         const CUtensorMap* mb = (seg == 1) ? &mapBs : &mapBb;
@@ -228,7 +154,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
             for (int c = 0; c < nchunk && ok; ++c) {
                 const int b = c & 1;
                 const uint32_t acc = tmem_d + (uint32_t)(b * TN);
-                if (!mbar_wait(acce0 + 8 * b, ((uint32_t)(c >> 1) & 1u) ^ 1u, limit)) break;   // buffer drained
+                if (!mbar_wait(acce0 + 8 * b, ((uint32_t)(c >> 1) & 1u) ^ 1u, limit, &g_tc_error)) break;   // buffer drained
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const int kb0 = c * CHUNK_KB, kb1 = min(P.nkb, kb0 + CHUNK_KB);
                 bool first = true;
@@ -236,7 +162,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
                     for (int kb = kb0; kb < kb1; ++kb, ++t) {
                         const int s = t % STAGES;
                         const uint32_t ph = (uint32_t)(t / STAGES) & 1u;
-                        if (!mbar_wait(full0 + 8 * s, ph, limit)) { ok = false; break; }
+                        if (!mbar_wait(full0 + 8 * s, ph, limit, &g_tc_error)) { ok = false; break; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint64_t da = smem_desc(base + s * STAGE_BYTES);
                         const uint64_t db = smem_desc(base + s * STAGE_BYTES + A_STAGE);
@@ -261,7 +187,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
         bool ok = true;
         for (int c = 0; c < nchunk; ++c) {
             const int b = c & 1;
-            ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (uint32_t)(c >> 1) & 1u, limit));   // warp-uniform
+            ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (uint32_t)(c >> 1) & 1u, limit, &g_tc_error));   // warp-uniform
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -296,23 +222,6 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(TMEM_COLS)
                      : "memory");
     }
-}
-
-using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                              const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeFn encode_fn() {
-    static EncodeFn fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        NC_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q));
-        if (!p || q != cudaDriverEntryPointSuccess)
-            throw Error(NC_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-        fn = reinterpret_cast<EncodeFn>(p);
-    }
-    return fn;
 }
 
 // rows x Kr floats (Kr contiguous, row stride ld floats), batch planes sbatch floats apart.
