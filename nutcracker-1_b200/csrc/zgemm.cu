@@ -13,6 +13,8 @@
 // cp.async stores and the 128-bit fragment loads are bank-conflict free:
 //   A, op N : As[k][m] (pitch BM+2)   A, op T/C : As[m][k] (pitch BK+4)
 //   B, op N : Bs[n][k] (pitch BK+4)   B, op T/C : Bs[k][n] (pitch BN+2)
+#include <algorithm>
+
 #include "nc_common.cuh"
 #include "nc_kernels.h"
 
@@ -207,12 +209,25 @@ void launch_cfg(const ZGemmParams& p, cudaStream_t s) {
 
 template <int OPA, int OPB>
 void launch_ops(const ZGemmParams& p, cudaStream_t s) {
-    // Large problems: 128x64 tiles, 8 warps; small ones: 64x64, 4 warps.
-    long long tiles128 = (long long)ceil_div(p.M, 128) * ceil_div(p.N, 64) * p.batch * p.nsplit;
-    if (p.M >= 128 && tiles128 >= 148)
-        launch_cfg<128, 64, 16, 32, 32, 3, OPA, OPB>(p, s);
-    else
-        launch_cfg<64, 64, 16, 32, 32, 3, OPA, OPB>(p, s);
+    // The tile whose busiest SM gets the least work: outputs per SM times a
+    // weight for the smaller tiles' lower reuse of shared memory (fitted to
+    // the times below).  Small products need small tiles to reach all SMs: on
+    // a B200 an H_eff product of a Heisenberg site takes, with 64x64 and
+    // 128x64 tiles only / with this rule, 61.8 / 17.7 us at bond dimension 48,
+    // 54.7 / 21.9 at 64, 62.0 / 35.2 at 128, 80.4 / 71.4 at 192.  The K order of an
+    // output does not depend on the tile, so neither do the results.
+    const long long z = (long long)p.batch * p.nsplit;
+    auto load = [&](int bm, int bn, double w) {
+        const long long t = (long long)ceil_div(p.M, bm) * ceil_div(p.N, bn) * z;
+        return (double)((t + 147) / 148) * bm * bn * w;
+    };
+    const double l16 = load(16, 16, 1.25), l32 = load(32, 32, 1.1), l64 = load(64, 64, 1.0);
+    const double l128 = p.M >= 128 ? load(128, 64, 0.95) : 1e30;
+    const double best = std::min(std::min(l16, l32), std::min(l64, l128));
+    if (best == l128) launch_cfg<128, 64, 16, 32, 32, 3, OPA, OPB>(p, s);
+    else if (best == l64) launch_cfg<64, 64, 16, 32, 32, 3, OPA, OPB>(p, s);
+    else if (best == l32) launch_cfg<32, 32, 32, 16, 16, 3, OPA, OPB>(p, s);
+    else launch_cfg<16, 16, 32, 8, 8, 3, OPA, OPB>(p, s);
 }
 
 // C[b] = alpha * sum_ks ws[ks][b] + beta * C[b]
