@@ -21,89 +21,61 @@
 
 #include "nc_common.cuh"
 #include "nc_kernels.h"
+#include "nc_mix.cuh"
 
 namespace nc {
 
 namespace {
 
-constexpr int MIX_MAX_NNZ = 64;
-constexpr int MIX_MAX_D = 4;
-
 // The sparse mixes.  Both are bound by HBM (each input element read once, each
 // output written once), so a block stages its inputs in shared memory, all
-// channels of RT consecutive elements, and makes every output of them from
+// channels of up to 128 consecutive elements, and makes every output of them from
 // there: read once per output instead (the first form), a chi=1024 Heisenberg
 // mix_left took 214 us on a B200 where its 336 MB take 51 us; this form takes
-// 108 us.  An operator with more channels than fit (MIX_MAX_STAGE
+// 75 us.  An operator with more channels than fit (MIX_MAX_STAGE
 // elements of one position) keeps the direct form, one thread per output.
 // The terms of an output are added in the order of the operator's matrices.
-constexpr int MIX_T = 256;
 constexpr int MIX_STAGE = 3072;        // elements staged per block (48 KiB)
-constexpr int MIX_MAX_STAGE = 384;     // channels x d at most: 8 positions per block
-
-// Matrices grouped by `to` (or `from`) index, in their own order within a group.
-struct MixTable {
-    cplx W[MIX_MAX_NNZ * MIX_MAX_D * MIX_MAX_D];
-    int other[MIX_MAX_NNZ];          // the other index of each matrix
-    int first[MIX_MAX_STAGE + 1];    // group k: matrices first[k] .. first[k+1] - 1
-};
-__device__ __forceinline__ void mix_table(MixTable& t, int nnz, int d, int groups, bool by_to, const uint32_t* __restrict__ idx,
-                                          const cplx* __restrict__ W) {
-    __shared__ int at[MIX_MAX_NNZ];
-    for (int n = threadIdx.x; n < nnz; n += blockDim.x) {
-        const int mine = (int)idx[2 * n + (by_to ? 1 : 0)];
-        int pos = 0;   // matrices with a smaller key, or the same key and earlier
-        for (int q = 0; q < nnz; ++q) {
-            const int k = (int)idx[2 * q + (by_to ? 1 : 0)];
-            pos += (k < mine || (k == mine && q < n)) ? 1 : 0;
-        }
-        at[n] = pos;
-        t.other[pos] = (int)idx[2 * n + (by_to ? 0 : 1)] - 1;
-    }
-    for (int k = threadIdx.x; k <= groups; k += blockDim.x) {
-        int pos = 0;
-        for (int q = 0; q < nnz; ++q) pos += ((int)idx[2 * q + (by_to ? 1 : 0)] - 1 < k) ? 1 : 0;
-        t.first[k] = pos;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nnz * d * d; i += blockDim.x) t.W[at[i / (d * d)] * d * d + i % (d * d)] = W[i];
-    __syncthreads();
-}
 
 // U(r,k2,j,b) = sum_{n: to(n)=k2} sum_a W(a,b,n) T(r,j,k1(n),a)
 template <int D>
-__global__ void __launch_bounds__(MIX_T) mix_left_staged_kernel(int br, int bl, int cl, int cr, int nnz, int rt,
+__global__ void __launch_bounds__(MIX_T) mix_left_staged_kernel(int br, int bl, int cl, int cr, int nnz, int lrt,
                                                                 const uint32_t* __restrict__ idx,
                                                                 const cplx* __restrict__ W,
                                                                 const cplx* __restrict__ T, cplx* __restrict__ U) {
     __shared__ MixTable tab;
     extern __shared__ __align__(16) unsigned char mix_smem[];
-    cplx* st = reinterpret_cast<cplx*>(mix_smem);   // [k1 + cl a][rt]
+    cplx* st = reinterpret_cast<cplx*>(mix_smem);   // [k1 + cl a][2^lrt]
     mix_table(tab, nnz, D, cr, true, idx, W);
-    const int rblocks = (br + rt - 1) / rt;
+    // a thread keeps its position; the channels go round the groups of threads
+    const int rt = 1 << lrt, grp = threadIdx.x >> lrt, ngrp = MIX_T >> lrt, r = threadIdx.x & (rt - 1);
+    const int rblocks = (br + rt - 1) >> lrt;
     const long long items = (long long)rblocks * bl;
     for (long long it = blockIdx.x; it < items; it += gridDim.x) {
-        const int j = (int)(it / rblocks), r0 = (int)(it % rblocks) * rt, nr = min(rt, br - r0);
-        for (int e = threadIdx.x; e < cl * D * rt; e += MIX_T) {
-            const int r = e % rt, ch = e / rt;
-            if (r < nr) st[e] = T[r0 + r + (long long)br * (j + (long long)bl * ch)];
-        }
+        const int j = (int)(it / rblocks), r0 = (int)(it % rblocks) << lrt;
+        if (r0 + r < br)
+            for (int ch = grp; ch < cl * D; ch += ngrp)
+                st[(ch << lrt) + r] = T[r0 + r + (long long)br * (j + (long long)bl * ch)];
         __syncthreads();
-        for (int e = threadIdx.x; e < cr * D * rt; e += MIX_T) {
-            const int r = e % rt, o = e / rt, k2 = o % cr, b = o / cr;
-            if (r >= nr) continue;
-            cplx acc = cmake(0, 0);
-            const int last = tab.first[k2 + 1];
-            for (int n = tab.first[k2]; n < last; ++n) {
-                const cplx* tk = st + tab.other[n] * rt + r;
+        if (r0 + r < br) {
+            int k2 = grp, b = 0;
+            while (k2 >= cr) { k2 -= cr; ++b; }
+            while (b < D) {
+                cplx acc = cmake(0, 0);
+                const int last = tab.first[k2 + 1];
+                for (int n = tab.first[k2]; n < last; ++n) {
+                    const cplx* tk = st + (tab.other[n] << lrt) + r;
 #pragma unroll
-                for (int a = 0; a < D; ++a) {
-                    const cplx w = tab.W[(n * D + b) * D + a];
-                    const cplx tv = tk[a * cl * rt];
-                    acc = cadd(acc, cmul(w, tv));
+                    for (int a = 0; a < D; ++a) {
+                        const cplx w = tab.W[(n * D + b) * D + a];
+                        const cplx tv = tk[(a * cl) << lrt];
+                        acc = cadd(acc, cmul(w, tv));
+                    }
                 }
+                U[r0 + r + (long long)br * (k2 + (long long)cr * (j + (long long)bl * b))] = acc;
+                k2 += ngrp;
+                while (k2 >= cr) { k2 -= cr; ++b; }
             }
-            U[r0 + r + (long long)br * (k2 + (long long)cr * (j + (long long)bl * b))] = acc;
         }
         __syncthreads();
     }
@@ -112,37 +84,47 @@ __global__ void __launch_bounds__(MIX_T) mix_left_staged_kernel(int br, int bl, 
 // Z(x,r,a,k1) = sum_{n: from(n)=k1} sum_b W(a,b,n) Y(x,b,r,k2(n)),
 // Y (bl,d,br,cr), Z (bl,br,d,cl).
 template <int D>
-__global__ void __launch_bounds__(MIX_T) mix_right_staged_kernel(int br, int bl, int cl, int cr, int nnz, int rt,
+__global__ void __launch_bounds__(MIX_T) mix_right_staged_kernel(int br, int bl, int cl, int cr, int nnz, int lrt,
                                                                  const uint32_t* __restrict__ idx,
                                                                  const cplx* __restrict__ W,
                                                                  const cplx* __restrict__ Y, cplx* __restrict__ Z) {
     __shared__ MixTable tab;
     extern __shared__ __align__(16) unsigned char mix_smem[];
-    cplx* st = reinterpret_cast<cplx*>(mix_smem);   // [k2 + cr b][rt]
+    cplx* st = reinterpret_cast<cplx*>(mix_smem);   // [k2 + cr b][2^lrt]
     mix_table(tab, nnz, D, cl, false, idx, W);
-    const int xblocks = (bl + rt - 1) / rt;
+    const int rt = 1 << lrt, grp = threadIdx.x >> lrt, ngrp = MIX_T >> lrt, x = threadIdx.x & (rt - 1);
+    const int xblocks = (bl + rt - 1) >> lrt;
     const long long items = (long long)xblocks * br;
     for (long long it = blockIdx.x; it < items; it += gridDim.x) {
-        const int r = (int)(it / xblocks), x0 = (int)(it % xblocks) * rt, nx = min(rt, bl - x0);
-        for (int e = threadIdx.x; e < cr * D * rt; e += MIX_T) {
-            const int x = e % rt, ch = e / rt, k2 = ch % cr, b = ch / cr;
-            if (x < nx) st[e] = Y[x0 + x + (long long)bl * (b + (long long)D * (r + (long long)br * k2))];
+        const int r = (int)(it / xblocks), x0 = (int)(it % xblocks) << lrt;
+        if (x0 + x < bl) {
+            int k2 = grp, b = 0;
+            while (k2 >= cr) { k2 -= cr; ++b; }
+            while (b < D) {
+                st[((k2 + cr * b) << lrt) + x] = Y[x0 + x + (long long)bl * (b + (long long)D * (r + (long long)br * k2))];
+                k2 += ngrp;
+                while (k2 >= cr) { k2 -= cr; ++b; }
+            }
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < cl * D * rt; e += MIX_T) {
-            const int x = e % rt, o = e / rt, k1 = o % cl, a = o / cl;
-            if (x >= nx) continue;
-            cplx acc = cmake(0, 0);
-            const int last = tab.first[k1 + 1];
-            for (int n = tab.first[k1]; n < last; ++n) {
-                const cplx* yk = st + tab.other[n] * rt + x;
+        if (x0 + x < bl) {
+            int k1 = grp, a = 0;
+            while (k1 >= cl) { k1 -= cl; ++a; }
+            while (a < D) {
+                cplx acc = cmake(0, 0);
+                const int last = tab.first[k1 + 1];
+                for (int n = tab.first[k1]; n < last; ++n) {
+                    const cplx* yk = st + (tab.other[n] << lrt) + x;
 #pragma unroll
-                for (int b = 0; b < D; ++b) {
-                    const cplx w = tab.W[(n * D + b) * D + a];
-                    acc = cadd(acc, cmul(w, yk[b * cr * rt]));
+                    for (int b = 0; b < D; ++b) {
+                        const cplx w = tab.W[(n * D + b) * D + a];
+                        acc = cadd(acc, cmul(w, yk[(b * cr) << lrt]));
+                    }
                 }
+                Z[x0 + x + (long long)bl * (r + (long long)br * (a + (long long)D * k1))] = acc;
+                k1 += ngrp;
+                while (k1 >= cl) { k1 -= cl; ++a; }
             }
-            Z[x0 + x + (long long)bl * (r + (long long)br * (a + (long long)D * k1))] = acc;
         }
         __syncthreads();
     }
@@ -234,42 +216,44 @@ void check_op(const MpoSite& op) {
     NC_ARG(op.cl >= 1 && op.cr >= 1, "MPO site: bond dimensions must be >= 1");
 }
 
-// Positions per block of the staged mixes: as many as fit, at most 128 (fewer
-// when that leaves SMs without a block); 0 when the direct form has to do it.
+// log2 of the positions per block of the staged mixes: as many as fit, at most
+// 128 (fewer when that leaves SMs without a block); -1 when the direct form
+// has to do it.
 int mix_positions(int in_channels, int out_channels, long long along, long long across) {
-    if (in_channels > MIX_MAX_STAGE || out_channels > MIX_MAX_STAGE) return 0;
-    int rt = std::min(128, MIX_STAGE / in_channels / 8 * 8);
-    while (rt > 32 && (rt >= 2 * along || (along + rt - 1) / rt * across < 2 * 148)) rt /= 2;
-    return std::max(8, rt / 8 * 8);
+    if (in_channels > MIX_MAX_STAGE || out_channels > MIX_MAX_STAGE) return -1;
+    int l = 7;
+    while (l > 3 && (in_channels << l) > MIX_STAGE) --l;
+    while (l > 5 && ((1 << l) >= 2 * along || ((along + (1 << l) - 1) >> l) * across < 2 * 148)) --l;
+    return l;
 }
 
 template <int D>
-void launch_mix_left_staged(cudaStream_t s, int rt, int bl, int br, const MpoSite& op, const cplx* T, cplx* U) {
+void launch_mix_left_staged(cudaStream_t s, int lrt, int bl, int br, const MpoSite& op, const cplx* T, cplx* U) {
     NC_SET_SMEM_ONCE(mix_left_staged_kernel<D>, sizeof(cplx) * MIX_STAGE);
-    const long long items = (long long)ceil_div(br, rt) * bl;
+    const long long items = (long long)ceil_div(br, 1 << lrt) * bl;
     mix_left_staged_kernel<D><<<(unsigned)std::min<long long>(items, 148 * 16), MIX_T,
-                                sizeof(cplx) * (size_t)rt * op.cl * D, s>>>(br, bl, op.cl, op.cr, op.nnz, rt, op.idx,
+                                sizeof(cplx) * ((size_t)op.cl * D << lrt), s>>>(br, bl, op.cl, op.cr, op.nnz, lrt, op.idx,
                                                                            op.W, T, U);
 }
 
 template <int D>
-void launch_mix_right_staged(cudaStream_t s, int rt, int bl, int br, const MpoSite& op, const cplx* Y, cplx* Z) {
+void launch_mix_right_staged(cudaStream_t s, int lrt, int bl, int br, const MpoSite& op, const cplx* Y, cplx* Z) {
     NC_SET_SMEM_ONCE(mix_right_staged_kernel<D>, sizeof(cplx) * MIX_STAGE);
-    const long long items = (long long)ceil_div(bl, rt) * br;
+    const long long items = (long long)ceil_div(bl, 1 << lrt) * br;
     mix_right_staged_kernel<D><<<(unsigned)std::min<long long>(items, 148 * 16), MIX_T,
-                                 sizeof(cplx) * (size_t)rt * op.cr * D, s>>>(br, bl, op.cl, op.cr, op.nnz, rt, op.idx,
+                                 sizeof(cplx) * ((size_t)op.cr * D << lrt), s>>>(br, bl, op.cl, op.cr, op.nnz, lrt, op.idx,
                                                                             op.W, Y, Z);
 }
 
 void launch_mix_left(cudaStream_t s, int bl, int br, const MpoSite& op, const cplx* T, cplx* U) {
-    const int rt = mix_positions(op.cl * op.d, op.cr * op.d, br, bl);
-    if (!rt)
+    const int lrt = mix_positions(op.cl * op.d, op.cr * op.d, br, bl);
+    if (lrt < 0)
         mix_left_kernel<<<grid_for((long long)br * op.cr * bl * op.d, 256), 256, 0, s>>>(br, bl, op.cl, op.cr, op.d,
                                                                                       op.nnz, op.idx, op.W, T, U);
-    else if (op.d == 1) launch_mix_left_staged<1>(s, rt, bl, br, op, T, U);
-    else if (op.d == 2) launch_mix_left_staged<2>(s, rt, bl, br, op, T, U);
-    else if (op.d == 3) launch_mix_left_staged<3>(s, rt, bl, br, op, T, U);
-    else launch_mix_left_staged<4>(s, rt, bl, br, op, T, U);
+    else if (op.d == 1) launch_mix_left_staged<1>(s, lrt, bl, br, op, T, U);
+    else if (op.d == 2) launch_mix_left_staged<2>(s, lrt, bl, br, op, T, U);
+    else if (op.d == 3) launch_mix_left_staged<3>(s, lrt, bl, br, op, T, U);
+    else launch_mix_left_staged<4>(s, lrt, bl, br, op, T, U);
     NC_CHECK_LAUNCH();
 }
 
@@ -280,14 +264,14 @@ void mix_left(Context& ctx, int bl, int br, const MpoSite& op, const cplx* T, cp
 
 void mix_right(Context& ctx, int bl, int br, const MpoSite& op, const cplx* Y, cplx* Z) {
     cudaStream_t s = ctx.stream;
-    const int rt = mix_positions(op.cr * op.d, op.cl * op.d, bl, br);
-    if (!rt)
+    const int lrt = mix_positions(op.cr * op.d, op.cl * op.d, bl, br);
+    if (lrt < 0)
         mix_right_kernel<<<grid_for((long long)bl * br * op.d * op.cl, 256), 256, 0, s>>>(
             br, bl, op.cl, op.cr, op.d, op.nnz, op.idx, op.W, Y, Z);
-    else if (op.d == 1) launch_mix_right_staged<1>(s, rt, bl, br, op, Y, Z);
-    else if (op.d == 2) launch_mix_right_staged<2>(s, rt, bl, br, op, Y, Z);
-    else if (op.d == 3) launch_mix_right_staged<3>(s, rt, bl, br, op, Y, Z);
-    else launch_mix_right_staged<4>(s, rt, bl, br, op, Y, Z);
+    else if (op.d == 1) launch_mix_right_staged<1>(s, lrt, bl, br, op, Y, Z);
+    else if (op.d == 2) launch_mix_right_staged<2>(s, lrt, bl, br, op, Y, Z);
+    else if (op.d == 3) launch_mix_right_staged<3>(s, lrt, bl, br, op, Y, Z);
+    else launch_mix_right_staged<4>(s, lrt, bl, br, op, Y, Z);
     NC_CHECK_LAUNCH();
     ctx.launches++;
 }

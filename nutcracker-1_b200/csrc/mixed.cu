@@ -14,6 +14,7 @@
 
 #include "nc_common.cuh"
 #include "nc_kernels.h"
+#include "nc_mix.cuh"
 
 namespace nc {
 
@@ -91,22 +92,103 @@ void split_rows(Context& ctx, int rows, int K, int batch, const cplx* X, long lo
     ctx.launches++;
 }
 
-constexpr int MIXM_MAX_NNZ = 64;
-constexpr int MIXM_MAX_D = 4;
-
 // Output strides (complex units) of a mixed-precision operand element.
 struct Out4 {
     long long s0, s1, s2, s3;
 };
 
+// One mix as positions (p, q) times channels.  Input channel (k, f), output
+// channel (group, e):
+//   left:  p = r, q = j, in (k1, a), out (k2, b);   right: p = x, q = r, in (k2, b), out (k1, a)
+//   out(p, q, group, e) = sum_{n of the group} sum_f W_n(e, f) in(p, q, k(n), f)
+// in FP64, written as a TF32 pair at complex offset p op + q oq + group og + e oe.
+struct MixTf32 {
+    int np, nq, kin, kout, nnz, lp, lq;      // positions, input and output channels, tile 2^lp x 2^lq
+    const uint32_t* idx;
+    const cplx* W;
+    const float2* in;
+    long long iq, ik, ie;                    // input strides of q, k, f (p contiguous)
+    float *ob, *os;
+    long long op, oq, og, oe;
+};
+
+constexpr int MIXT_BYTES = 48 * 1024;        // staged channels of one tile
+
+// The mix is bound by HBM, but reads along p and, depending on the operand it
+// makes, writes along p or along q.  A block stages all channels of a tile of
+// positions (128 x 1, or square when the output runs along q, so that reads
+// and writes are both whole lines) and makes every output from shared memory.
+// On a B200, against one thread per output straight from global memory:
+// chi = 1024 Heisenberg product 175 -> 86 us, chi = 512 spin-1 right
+// environment, whose output is transposed, 102 -> 46 us.
+template <int D, bool RIGHT>
+__global__ void __launch_bounds__(MIX_T) mix_tf32_staged_kernel(MixTf32 P) {
+    __shared__ MixTable tab;
+    extern __shared__ __align__(16) unsigned char mixt_smem[];
+    float2* st = reinterpret_cast<float2*>(mixt_smem);   // [f][k][q][p], rows of pitch tp | 1
+    mix_table(tab, P.nnz, D, P.kout, !RIGHT, P.idx, P.W);
+    // a thread keeps its position in the tile; the channels go round the groups of threads
+    const int lp = P.lp, lq = P.lq, tp = 1 << lp, tq = 1 << lq, pitch = tp | 1, chan = pitch << lq;
+    const int grp = threadIdx.x >> (lp + lq), ngrp = MIX_T >> (lp + lq), pos = threadIdx.x & ((1 << (lp + lq)) - 1);
+    const bool along_p = P.op == 1;
+    const int pi = pos & (tp - 1), qi = pos >> lp;                                          // read along p
+    const int po = along_p ? pi : pos >> lq, qo = along_p ? qi : pos & (tq - 1);            // write along p or q
+    const int pblocks = (P.np + tp - 1) >> lp, qblocks = (P.nq + tq - 1) >> lq;
+    for (int it = blockIdx.x; it < pblocks * qblocks; it += gridDim.x) {
+        const int p0 = (it % pblocks) << lp, q0 = (it / pblocks) << lq;
+        if (p0 + pi < P.np && q0 + qi < P.nq) {
+            const float2* src = P.in + p0 + pi + (q0 + qi) * P.iq;
+            int k = grp, f = 0;
+            while (k >= P.kin) { k -= P.kin; ++f; }
+            while (f < D) {
+                st[(f * P.kin + k) * chan + qi * pitch + pi] = src[k * P.ik + f * P.ie];
+                k += ngrp;
+                while (k >= P.kin) { k -= P.kin; ++f; }
+            }
+        }
+        __syncthreads();
+        if (p0 + po < P.np && q0 + qo < P.nq) {
+            const float2* mine = st + qo * pitch + po;
+            const long long base = (p0 + po) * P.op + (q0 + qo) * P.oq;
+            int g = grp, e = 0;
+            while (g >= P.kout) { g -= P.kout; ++e; }
+            while (e < D) {
+                double ar = 0, ai = 0;
+                const int last = tab.first[g + 1];
+                for (int n = tab.first[g]; n < last; ++n) {
+                    const float2* x = mine + tab.other[n] * chan;
+#pragma unroll
+                    for (int f = 0; f < D; ++f) {
+                        const cplx w = RIGHT ? tab.W[(n * D + f) * D + e] : tab.W[(n * D + e) * D + f];
+                        const float2 t = x[f * P.kin * chan];
+                        ar += w.x * (double)t.x - w.y * (double)t.y;
+                        ai += w.x * (double)t.y + w.y * (double)t.x;
+                    }
+                }
+                float brr, bii, srr, sii;
+                split_tf32(ar, brr, srr);
+                split_tf32(ai, bii, sii);
+                const long long off = 2 * (base + g * P.og + e * P.oe);
+                *reinterpret_cast<float2*>(P.ob + off) = make_float2(brr, bii);
+                *reinterpret_cast<float2*>(P.os + off) = make_float2(srr, sii);
+                g += ngrp;
+                while (g >= P.kout) { g -= P.kout; ++e; }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// The direct forms: one thread per output, for operators with more channels
+// than a tile's shared memory holds.
 // U(r,k2,j,b) = sum_{n: to(n)=k2} sum_a W(a,b,n) T(r, j + bl*(k1(n) + cl*a))
 // (T complex64 from stage A), accumulated in FP64 and written as a TF32
 // pair at complex offset r*o.s0 + k2*o.s1 + j*o.s2 + b*o.s3.
 __global__ void mix_left_tf32_kernel(int br, int bl, int cl, int cr, int d, int nnz, const uint32_t* __restrict__ idx,
                                      const cplx* __restrict__ W, const float2* __restrict__ T,
                                      float* __restrict__ Ub, float* __restrict__ Us, Out4 o) {
-    __shared__ cplx Ws[MIXM_MAX_NNZ * MIXM_MAX_D * MIXM_MAX_D];
-    __shared__ int k1s[MIXM_MAX_NNZ], k2s[MIXM_MAX_NNZ];
+    __shared__ cplx Ws[MIX_MAX_NNZ * MIX_MAX_D * MIX_MAX_D];
+    __shared__ int k1s[MIX_MAX_NNZ], k2s[MIX_MAX_NNZ];
     for (int i = threadIdx.x; i < nnz * d * d; i += blockDim.x) Ws[i] = W[i];
     for (int i = threadIdx.x; i < nnz; i += blockDim.x) {
         k1s[i] = (int)idx[2 * i] - 1;
@@ -149,8 +231,8 @@ __global__ void mix_left_tf32_kernel(int br, int bl, int cl, int cr, int d, int 
 __global__ void mix_right_tf32_kernel(int br, int bl, int cl, int cr, int d, int nnz, const uint32_t* __restrict__ idx,
                                       const cplx* __restrict__ W, const float2* __restrict__ Y,
                                       float* __restrict__ Zb, float* __restrict__ Zs, Out4 o) {
-    __shared__ cplx Ws[MIXM_MAX_NNZ * MIXM_MAX_D * MIXM_MAX_D];
-    __shared__ int k1s[MIXM_MAX_NNZ], k2s[MIXM_MAX_NNZ];
+    __shared__ cplx Ws[MIX_MAX_NNZ * MIX_MAX_D * MIX_MAX_D];
+    __shared__ int k1s[MIX_MAX_NNZ], k2s[MIX_MAX_NNZ];
     for (int i = threadIdx.x; i < nnz * d * d; i += blockDim.x) Ws[i] = W[i];
     for (int i = threadIdx.x; i < nnz; i += blockDim.x) {
         k1s[i] = (int)idx[2 * i] - 1;
@@ -192,6 +274,66 @@ unsigned grid_for(long long total, int threads) {
     return (unsigned)std::max<long long>(1, std::min<long long>(g, 148 * 32));
 }
 
+template <int D, bool RIGHT>
+void launch_mix_tf32(Context& ctx, MixTf32& P) {
+    NC_SET_SMEM_ONCE((mix_tf32_staged_kernel<D, RIGHT>), MIXT_BYTES);
+    const long long tiles = (long long)ceil_div(P.np, 1 << P.lp) * ceil_div(P.nq, 1 << P.lq);
+    mix_tf32_staged_kernel<D, RIGHT><<<(unsigned)std::min<long long>(tiles, 148 * 16), MIX_T,
+                                       sizeof(float2) * (size_t)P.kin * D * (((1 << P.lp) | 1) << P.lq), ctx.stream>>>(
+        P);
+}
+
+// Picks the tile; false when the channels do not fit.
+template <bool RIGHT>
+bool mix_tf32_staged(Context& ctx, int d, MixTf32& P) {
+    const int cin = P.kin * d;
+    if (cin > MIX_MAX_STAGE || P.kout * d > MIX_MAX_STAGE) return false;
+    auto fits = [&] { return sizeof(float2) * (size_t)cin * (((1 << P.lp) | 1) << P.lq) <= (size_t)MIXT_BYTES; };
+    if (P.op == 1) {
+        P.lq = 0;
+        for (P.lp = 7; P.lp > 3 && !fits(); --P.lp) {}
+        while (P.lp > 5 && (long long)ceil_div(P.np, 1 << P.lp) * P.nq < 2 * 148) --P.lp;
+    } else {
+        for (P.lp = P.lq = 4; P.lp > 2 && !fits();) P.lp = P.lq = P.lp - 1;
+    }
+    if (!fits() || (long long)ceil_div(P.np, 1 << P.lp) * ceil_div(P.nq, 1 << P.lq) >= (1LL << 31)) return false;
+    if (d == 1) launch_mix_tf32<1, RIGHT>(ctx, P);
+    else if (d == 2) launch_mix_tf32<2, RIGHT>(ctx, P);
+    else if (d == 3) launch_mix_tf32<3, RIGHT>(ctx, P);
+    else launch_mix_tf32<4, RIGHT>(ctx, P);
+    return true;
+}
+
+// U from T (br, bl, cl, d) complex64; output strides o of (r, k2, j, b).
+void mix_left_tf32(Context& ctx, int bl, int br, const MpoSite& op, const float2* T, float* Ub, float* Us, Out4 o) {
+    MixTf32 P;
+    P.np = br; P.nq = bl; P.kin = op.cl; P.kout = op.cr; P.nnz = op.nnz; P.idx = op.idx; P.W = op.W;
+    P.in = T; P.iq = br; P.ik = (long long)br * bl; P.ie = (long long)br * bl * op.cl;
+    P.ob = Ub; P.os = Us; P.op = o.s0; P.oq = o.s2; P.og = o.s1; P.oe = o.s3;
+    if (!mix_tf32_staged<false>(ctx, op.d, P)) {
+        const long long total = (long long)br * op.cr * bl * op.d;
+        mix_left_tf32_kernel<<<grid_for(total, 256), 256, 0, ctx.stream>>>(br, bl, op.cl, op.cr, op.d, op.nnz, op.idx,
+                                                                           op.W, T, Ub, Us, o);
+    }
+    NC_CHECK_LAUNCH();
+    ctx.launches++;
+}
+
+// Z from Y (bl, d, br, cr) complex64; output strides o of (x, r, a, k1).
+void mix_right_tf32(Context& ctx, int bl, int br, const MpoSite& op, const float2* Y, float* Zb, float* Zs, Out4 o) {
+    MixTf32 P;
+    P.np = bl; P.nq = br; P.kin = op.cr; P.kout = op.cl; P.nnz = op.nnz; P.idx = op.idx; P.W = op.W;
+    P.in = Y; P.iq = (long long)bl * op.d; P.ik = (long long)bl * op.d * br; P.ie = bl;
+    P.ob = Zb; P.os = Zs; P.op = o.s0; P.oq = o.s1; P.og = o.s3; P.oe = o.s2;
+    if (!mix_tf32_staged<true>(ctx, op.d, P)) {
+        const long long total = (long long)bl * br * op.d * op.cl;
+        mix_right_tf32_kernel<<<grid_for(total, 256), 256, 0, ctx.stream>>>(br, bl, op.cl, op.cr, op.d, op.nnz, op.idx,
+                                                                            op.W, Y, Zb, Zs, o);
+    }
+    NC_CHECK_LAUNCH();
+    ctx.launches++;
+}
+
 }  // namespace
 
 // ---- layout of one MixedHeff buffer ----------------------------------------
@@ -227,7 +369,7 @@ size_t mixed_heff_floats(int bl, int br, const MpoSite& op) { return mixed_layou
 
 void mixed_heff_prepare(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L, const cplx* R,
                         float* buf, MixedHeff* h) {
-    NC_ARG(op.nnz >= 1 && op.nnz <= MIXM_MAX_NNZ && op.d >= 1 && op.d <= MIXM_MAX_D,
+    NC_ARG(op.nnz >= 1 && op.nnz <= MIX_MAX_NNZ && op.d >= 1 && op.d <= MIX_MAX_D,
            "mixed H_eff: nnz must be in [1,64] and d in [1,4]");
     const MixedLayout s = mixed_layout(bl, br, op);
     h->bl = bl; h->br = br; h->op = op;
@@ -253,12 +395,8 @@ void heff_apply_mixed(Context& ctx, const MixedHeff& h, const cplx* x, cplx* y) 
     ga.M = br; ga.Nr = 2 * bl * cl; ga.Kr = 2 * bl; ga.batch = d;
     ga.C = h.T; ga.sm = 1; ga.sn = br; ga.sz = (long long)br * bl * cl; ga.c_fp64 = false;
     tc_gemm(ctx, ga);
-    const long long total = (long long)br * cr * bl * d;
-    const Out4 o = {1, br, h.ldU / 2, (long long)bl * (h.ldU / 2)};   // row (b, j), K index r + br*k2
-    mix_left_tf32_kernel<<<grid_for(total, 256), 256, 0, ctx.stream>>>(br, bl, cl, cr, d, h.op.nnz, h.op.idx,
-                                                                       h.op.W, h.T, h.Ub, h.Us, o);
-    NC_CHECK_LAUNCH();
-    ctx.launches++;
+    // row (b, j), K index r + br*k2
+    mix_left_tf32(ctx, bl, br, h.op, h.T, h.Ub, h.Us, {1, br, h.ldU / 2, (long long)bl * (h.ldU / 2)});
     TcGemm gc;
     gc.A.big = h.Ub; gc.A.small = h.Us; gc.A.ld = h.ldU; gc.A.sbatch = (long long)bl * h.ldU;
     gc.B.big = h.Rb; gc.B.small = h.Rs; gc.B.ld = h.ldR; gc.B.sbatch = 0;
@@ -278,7 +416,7 @@ void expectation_mixed(Context& ctx, const MixedHeff& h, const cplx* psi, cplx* 
 // contract_sos_left (core.f95:623-677) in the precision form:
 // L'_{k2}(r,r'') = sum_{(j,b)} U(r,k2,j,b) conj(psi(r'',j,b)), U = mix(psi_a L).
 void sos_left_mixed(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L, const cplx* psi, cplx* Lnew) {
-    NC_ARG(op.nnz >= 1 && op.nnz <= MIXM_MAX_NNZ && op.d >= 1 && op.d <= MIXM_MAX_D,
+    NC_ARG(op.nnz >= 1 && op.nnz <= MIX_MAX_NNZ && op.d >= 1 && op.d <= MIX_MAX_D,
            "mixed environment: nnz must be in [1,64] and d in [1,4]");
     const int d = op.d, cl = op.cl, cr = op.cr;
     ArenaFrame f(ctx.arena);
@@ -301,12 +439,7 @@ void sos_left_mixed(Context& ctx, int bl, int br, const MpoSite& op, const cplx*
     ga.C = T; ga.sm = 1; ga.sn = br; ga.sz = (long long)br * bl * cl; ga.c_fp64 = false;
     tc_gemm(ctx, ga);
     // U_op[k2][r][(j + bl*b)]
-    const Out4 o = {ldS / 2, (long long)br * (ldS / 2), 1, bl};
-    const long long total = (long long)br * cr * bl * d;
-    mix_left_tf32_kernel<<<grid_for(total, 256), 256, 0, ctx.stream>>>(br, bl, cl, cr, d, op.nnz, op.idx, op.W, T,
-                                                                       Ub, Us, o);
-    NC_CHECK_LAUNCH();
-    ctx.launches++;
+    mix_left_tf32(ctx, bl, br, op, T, Ub, Us, {ldS / 2, (long long)br * (ldS / 2), 1, bl});
     // B(k = j + bl*b, r'') = conj(psi[r'' + br*k]): expanded rows r''
     split_rows<true, true>(ctx, br, bl * d, 1, psi, 1, br, 0, Pb, Ps, ldS, 0);
     TcGemm gc;
@@ -320,7 +453,7 @@ void sos_left_mixed(Context& ctx, int bl, int br, const MpoSite& op, const cplx*
 // contract_sos_right (core.f95:679-848) in the precision form:
 // Y = Psi^H R, Z = mix_right(Y), R'_{k1}(x,x') = sum_{(r,a)} Z(x,r,a,k1) psi(r,x',a).
 void sos_right_mixed(Context& ctx, int bl, int br, const MpoSite& op, const cplx* R, const cplx* psi, cplx* Rnew) {
-    NC_ARG(op.nnz >= 1 && op.nnz <= MIXM_MAX_NNZ && op.d >= 1 && op.d <= MIXM_MAX_D,
+    NC_ARG(op.nnz >= 1 && op.nnz <= MIX_MAX_NNZ && op.d >= 1 && op.d <= MIX_MAX_D,
            "mixed environment: nnz must be in [1,64] and d in [1,4]");
     const int d = op.d, cl = op.cl, cr = op.cr;
     ArenaFrame f(ctx.arena);
@@ -344,12 +477,7 @@ void sos_right_mixed(Context& ctx, int bl, int br, const MpoSite& op, const cplx
     gy.C = Y; gy.sm = 1; gy.sn = (long long)bl * d; gy.sz = 0; gy.c_fp64 = false;
     tc_gemm(ctx, gy);
     // Z_op[k1][x][(r + br*a)]
-    const Out4 o = {ldZ / 2, 1, br, (long long)bl * (ldZ / 2)};
-    const long long total = (long long)bl * br * d * cl;
-    mix_right_tf32_kernel<<<grid_for(total, 256), 256, 0, ctx.stream>>>(br, bl, cl, cr, d, op.nnz, op.idx, op.W, Y,
-                                                                        Zb, Zs, o);
-    NC_CHECK_LAUNCH();
-    ctx.launches++;
+    mix_right_tf32(ctx, bl, br, op, Y, Zb, Zs, {ldZ / 2, 1, br, (long long)bl * (ldZ / 2)});
     // B(k = r + br*a, x') = psi[r + br*x' + br*bl*a]: expanded rows x', one K block of 2*br floats per a
     split_rows<true>(ctx, bl, br, d, psi, br, 1, (long long)br * bl, Pb, Ps, ldZ, 2LL * br);
     TcGemm gr;
