@@ -127,6 +127,10 @@ struct Context {
     bool blocking_sync = false;
     cudaEvent_t sync_event = nullptr;
     void sync();
+    // Second stream of the site solver (created at its first use): the
+    // projected problem of one Lanczos step beside the next step's product.
+    cudaStream_t ritz_stream = nullptr;
+    cudaEvent_t ritz_ready = nullptr, ritz_done = nullptr;
     Context();
     ~Context();
     static Context& get();   // thread-local default context

@@ -108,6 +108,9 @@ void Context::sync() {
 
 Context::~Context() {
     if (sync_event) cudaEventDestroy(sync_event);
+    if (ritz_stream) cudaStreamDestroy(ritz_stream);
+    if (ritz_ready) cudaEventDestroy(ritz_ready);
+    if (ritz_done) cudaEventDestroy(ritz_done);
     if (red_counter) cudaFree(red_counter);
     if (own_stream) cudaStreamDestroy(own_stream);
     if (pinned) cudaFreeHost(pinned);
