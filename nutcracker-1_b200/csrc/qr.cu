@@ -14,7 +14,8 @@
 // to 16 CTAs with the block held in registers (mp <= 2048 rows); devices
 // that cannot co-schedule such a cluster use inner panels of JB=4 columns
 // (one CTA each) and a per-column update kernel.  Q is formed explicitly by
-// backward accumulation of the block reflectors (zungqr order).
+// backward accumulation of the block reflectors (zungqr order) or, in the
+// look-ahead form, from the compact-WY factor of all of them.
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -235,10 +236,8 @@ __global__ void __launch_bounds__(PT) panel_apply_kernel(int mp, int jb, const c
 constexpr int BT_T = 1024;
 constexpr size_t BT_SMEM = sizeof(cplx) * ((size_t)2 * NB * (NB + 1) + NB * NB / 2);
 
-// G is either a matrix (ld nb) or, with nparts > 0, the sum of nparts NB x NB
-// partial Gram blocks (ld NB, stride NB*NB) added in index order.
-__global__ void __launch_bounds__(BT_T) build_t_kernel(int nb, const cplx* __restrict__ G, int nparts,
-                                                      const cplx* __restrict__ tau, cplx* __restrict__ T,
+// G: ld nb.
+__global__ void __launch_bounds__(BT_T) build_t_kernel(int nb, const cplx* __restrict__ G, const cplx* __restrict__ tau, cplx* __restrict__ T,
                                                       int ldt) {
     extern __shared__ __align__(16) unsigned char bt_smem[];
     cplx* Ts = reinterpret_cast<cplx*>(bt_smem);   // [NB][NB+1]
@@ -248,24 +247,7 @@ __global__ void __launch_bounds__(BT_T) build_t_kernel(int nb, const cplx* __res
     for (int e = tid; e < NB * NB; e += BT_T) {
         const int i = e % NB, j = e / NB;
         cplx g = cmake(0, 0);
-        if (i < j && j < nb) {
-            if (nparts > 0) {
-                double r0 = 0, i0 = 0, r1 = 0, i1 = 0;   // two interleaved chains, fixed order
-                int c = 0;
-                for (; c + 1 < nparts; c += 2) {
-                    const cplx a = G[(size_t)c * NB * NB + i + NB * j];
-                    const cplx b = G[(size_t)(c + 1) * NB * NB + i + NB * j];
-                    r0 += a.x; i0 += a.y; r1 += b.x; i1 += b.y;
-                }
-                if (c < nparts) {
-                    const cplx a = G[(size_t)c * NB * NB + i + NB * j];
-                    r0 += a.x; i0 += a.y;
-                }
-                g = cmake(r0 + r1, i0 + i1);
-            } else {
-                g = G[i + (long long)nb * j];
-            }
-        }
+        if (i < j && j < nb) g = G[i + (long long)nb * j];
         Gs[i * (NB + 1) + j] = g;
         Ts[i * (NB + 1) + j] = (i == j && i < nb) ? tau[i] : cmake(0, 0);
     }
@@ -303,162 +285,73 @@ __global__ void __launch_bounds__(BT_T) build_t_kernel(int nb, const cplx* __res
     }
 }
 
-void launch_build_t(Context& ctx, int nb, const cplx* G, const cplx* tau, cplx* T, int nparts = 0) {
+void launch_build_t(Context& ctx, int nb, const cplx* G, const cplx* tau, cplx* T) {
     NC_SET_SMEM_ONCE(build_t_kernel, BT_SMEM);
-    build_t_kernel<<<1, BT_T, BT_SMEM, ctx.stream>>>(nb, G, nparts, tau, T, NB);
+    build_t_kernel<<<1, BT_T, BT_SMEM, ctx.stream>>>(nb, G, tau, T, NB);
     NC_CHECK_LAUNCH();
     ctx.launches++;
 }
 
-// ---------------------------------------------------------------------------
-// One block reflector applied to one block of at most NB columns,
-//   C <- (I - V T V^H)^H C = C - V T^H (V^H C)     (V mp x nb, C mp x nc),
-// and the Gram matrix V^H V of the block, for the critical path of the
-// look-ahead QR.  The products are small (64 x 64 outputs, K = mp <= 2048),
-// so instead of split-K GEMMs on a handful of tiles they run as
-//   refl_partial_kernel: per 32-row chunk, the 64 x 64 partial of V^H C
-//                        (one CTA per chunk, operands staged in shared memory);
-//   refl_w2_kernel:      per column k, the chunk partials summed in chunk order
-//                        and W2(:,k) = T^H W(:,k);
-//   refl_apply_kernel:   per 32-row chunk, C -= V W2.
-// The Gram matrix is refl_partial_kernel with C = V, its partials summed by
-// build_t_kernel.  Every sum runs in a fixed order (bit-reproducible).
-// ---------------------------------------------------------------------------
-constexpr int RC = 32;                                     // rows per chunk
-constexpr int RT = 256;                                    // threads
-constexpr int RL = NB + 1;                                 // padded shared-memory row
-constexpr size_t RP_SMEM = sizeof(cplx) * 2 * RC * RL;     // V and C chunks
-constexpr size_t RA_SMEM = sizeof(cplx) * (NB + RC) * RL;  // W2 and the V chunk
-
-__global__ void __launch_bounds__(RT) refl_partial_kernel(int mp, int nb, const cplx* __restrict__ V, long long ldv,
-                                                          const cplx* __restrict__ C, long long ldc, int nc,
-                                                          cplx* __restrict__ part) {
-    extern __shared__ __align__(16) unsigned char rp_smem[];
-    cplx* Vs = reinterpret_cast<cplx*>(rp_smem);   // [RC][RL]
-    cplx* Cs = Vs + RC * RL;                         // [RC][RL]
-    const int r0 = blockIdx.x * RC, tid = threadIdx.x;
-    for (int e = tid; e < RC * NB; e += RT) {
-        const int r = e % RC, c = e / RC, row = r0 + r;
-        Vs[r * RL + c] = (row < mp && c < nb) ? V[row + ldv * c] : cmake(0, 0);
-        Cs[r * RL + c] = (row < mp && c < nc) ? C[row + ldc * c] : cmake(0, 0);
-    }
+// W2 = T^H W (nb x nc) without forming T: T^-H = diag(1 / conj(tau)) + the strict
+// lower part of V^H V (the compact-WY identity T^-1 + T^-H = V^H V), so W2 comes
+// out of a forward substitution, one warp per column and G = V^H V in shared
+// memory.  64 dependent steps, 8 us on a B200, where building T takes 27 us and
+// multiplying by it another 14.
+constexpr int TRS_WARPS = 4;
+constexpr size_t TRS_SMEM = sizeof(cplx) * NB * NB;
+__global__ void __launch_bounds__(32 * TRS_WARPS) reflector_solve_kernel(int nb, int nc, const cplx* __restrict__ G,
+                                                                         const cplx* __restrict__ tau,
+                                                                         const cplx* __restrict__ W,
+                                                                         cplx* __restrict__ W2) {
+    extern __shared__ __align__(16) unsigned char trs_smem[];
+    cplx* Gs = reinterpret_cast<cplx*>(trs_smem);   // column-major, ld nb
+    __shared__ cplx ts[NB];
+    for (int e = threadIdx.x; e < nb * nb; e += 32 * TRS_WARPS) Gs[e] = G[e];
+    for (int e = threadIdx.x; e < nb; e += 32 * TRS_WARPS) ts[e] = cconj(tau[e]);
     __syncthreads();
-    const int k = tid % NB, i0 = (tid / NB) * (NB / 4);   // 16 outputs (i0..i0+15, k) per thread
-    double ar[NB / 4], ai[NB / 4];
-#pragma unroll
-    for (int q = 0; q < NB / 4; ++q) ar[q] = ai[q] = 0;
-    for (int r = 0; r < RC; ++r) {
-        const cplx c = Cs[r * RL + k];
-#pragma unroll
-        for (int q = 0; q < NB / 4; ++q) {
-            const cplx v = Vs[r * RL + i0 + q];   // conj(v) * c
-            ar[q] = fma(v.x, c.x, fma(v.y, c.y, ar[q]));
-            ai[q] = fma(v.x, c.y, fma(-v.y, c.x, ai[q]));
-        }
-    }
-    cplx* out = part + (size_t)blockIdx.x * NB * NB;
-#pragma unroll
-    for (int q = 0; q < NB / 4; ++q) out[i0 + q + NB * k] = cmake(ar[q], ai[q]);
-}
-
-__global__ void __launch_bounds__(RT) refl_w2_kernel(int nparts, int nb, const cplx* __restrict__ part,
-                                                     const cplx* __restrict__ T, int ldt, cplx* __restrict__ W2) {
-    __shared__ cplx red[RT / NB][NB];
-    __shared__ cplx Ws[NB];
-    const int k = blockIdx.x, tid = threadIdx.x, i = tid % NB, q = tid / NB;
-    double sr = 0, si = 0;
-    for (int c = q; c < nparts; c += RT / NB) {
-        const cplx a = part[(size_t)c * NB * NB + i + NB * k];
-        sr += a.x;
-        si += a.y;
-    }
-    red[q][i] = cmake(sr, si);
-    __syncthreads();
-    if (q == 0) {
-        cplx w = red[0][i];
-#pragma unroll
-        for (int g = 1; g < RT / NB; ++g) w = cadd(w, red[g][i]);
-        Ws[i] = w;
-    }
-    __syncthreads();
-    if (q == 0) {
-        // W2(i,k) = sum_{l <= i} conj(T(l,i)) W(l,k)   (T upper triangular)
-        double wr = 0, wi = 0;
-        if (i < nb)
-            for (int l = 0; l <= i; ++l) {
-                const cplx t = T[l + (long long)ldt * i], w = Ws[l];
-                wr = fma(t.x, w.x, fma(t.y, w.y, wr));
-                wi = fma(t.x, w.y, fma(-t.y, w.x, wi));
-            }
-        W2[i + NB * k] = cmake(wr, wi);
-    }
-}
-
-__global__ void __launch_bounds__(RT) refl_apply_kernel(int mp, int nb, const cplx* __restrict__ V, long long ldv,
-                                                        const cplx* __restrict__ W2, cplx* __restrict__ C,
-                                                        long long ldc, int nc) {
-    extern __shared__ __align__(16) unsigned char ra_smem[];
-    cplx* Ws = reinterpret_cast<cplx*>(ra_smem);   // [NB][RL]: Ws[l * RL + k] = W2(l,k)
-    cplx* Vs = Ws + NB * RL;                         // [RC][RL]
-    const int r0 = blockIdx.x * RC, tid = threadIdx.x;
-    for (int e = tid; e < NB * NB; e += RT) {
-        const int l = e % NB, kk = e / NB;
-        Ws[l * RL + kk] = (l < nb && kk < nc) ? W2[l + NB * kk] : cmake(0, 0);
-    }
-    for (int e = tid; e < RC * NB; e += RT) {
-        const int r = e % RC, c = e / RC, row = r0 + r;
-        Vs[r * RL + c] = (row < mp && c < nb) ? V[row + ldv * c] : cmake(0, 0);
-    }
-    __syncthreads();
-    const int k = tid % NB, rq = (tid / NB) * (RC / 4);   // rows rq..rq+7 of column k
+    const int lane = threadIdx.x & 31, k = blockIdx.x * TRS_WARPS + (threadIdx.x >> 5);
     if (k >= nc) return;
-    double ar[RC / 4], ai[RC / 4];
-#pragma unroll
-    for (int q = 0; q < RC / 4; ++q) ar[q] = ai[q] = 0;
-    for (int l = 0; l < NB; ++l) {
-        const cplx w = Ws[l * RL + k];
-#pragma unroll
-        for (int q = 0; q < RC / 4; ++q) {
-            const cplx v = Vs[(rq + q) * RL + l];
-            ar[q] = fma(v.x, w.x, fma(-v.y, w.y, ar[q]));
-            ai[q] = fma(v.x, w.y, fma(v.y, w.x, ai[q]));
-        }
+    cplx w0 = lane < nb ? W[lane + (long long)nb * k] : cmake(0, 0);
+    cplx w1 = lane + 32 < nb ? W[lane + 32 + (long long)nb * k] : cmake(0, 0);
+    for (int i = 0; i < nb; ++i) {
+        const cplx own = i < 32 ? w0 : w1;
+        cplx v = cmake(__shfl_sync(0xffffffffu, own.x, i & 31), __shfl_sync(0xffffffffu, own.y, i & 31));
+        v = cmul(ts[i], v);
+        const cplx* g = Gs + i * nb;
+        if (lane == i) w0 = v;
+        else if (lane > i && lane < nb) w0 = csub(w0, cmul(g[lane], v));
+        if (lane + 32 == i) w1 = v;
+        else if (lane + 32 > i && lane + 32 < nb) w1 = csub(w1, cmul(g[lane + 32], v));
     }
-#pragma unroll
-    for (int q = 0; q < RC / 4; ++q) {
-        const int row = r0 + rq + q;
-        if (row < mp) {
-            cplx& c = C[row + ldc * k];
-            c = cmake(c.x - ar[q], c.y - ai[q]);
-        }
+    if (lane < nb) W2[lane + (long long)nb * k] = w0;
+    if (lane + 32 < nb) W2[lane + 32 + (long long)nb * k] = w1;
+}
+
+// Zeros above the diagonal blocks of V (columns c, rows < NB floor(c / NB)) and
+// in the whole of T (n x n).
+__global__ void zero_upper_kernel(int n, cplx* __restrict__ V, long long ldv, cplx* __restrict__ T) {
+    const long long total = (long long)n * n;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
+         e += (long long)gridDim.x * blockDim.x) {
+        const int r = (int)(e % n), c = (int)(e / n);
+        T[e] = cmake(0, 0);
+        if (r < c / NB * NB) V[r + c * ldv] = cmake(0, 0);
     }
 }
 
-int refl_chunks(int mp) { return (mp + RC - 1) / RC; }
-
-void refl_attrs() {
-    NC_SET_SMEM_ONCE(refl_partial_kernel, RP_SMEM);
-    NC_SET_SMEM_ONCE(refl_apply_kernel, RA_SMEM);
+// The nb x nb block T (ld NB) to the diagonal of the full factor (ld n).
+__global__ void place_t_kernel(int nb, const cplx* __restrict__ T, cplx* __restrict__ full, long long ldf) {
+    for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) full[e % nb + (e / nb) * ldf] = T[e % nb + NB * (e / nb)];
 }
 
-// part (refl_chunks(mp) x NB x NB) = chunk partials of V^H C.
-void launch_refl_partial(Context& ctx, int mp, int nb, const cplx* V, long long ldv, const cplx* C, long long ldc,
-                         int nc, cplx* part) {
-    refl_attrs();
-    refl_partial_kernel<<<refl_chunks(mp), RT, RP_SMEM, ctx.stream>>>(mp, nb, V, ldv, C, ldc, nc, part);
-    NC_CHECK_LAUNCH();
-    ctx.launches++;
-}
-
-// C -= V T^H (V^H C), from the chunk partials of V^H C.
-void launch_refl_finish(Context& ctx, int mp, int nb, const cplx* V, long long ldv, const cplx* T, int ldt,
-                        const cplx* part, cplx* W2, cplx* C, long long ldc, int nc) {
-    refl_attrs();
-    refl_w2_kernel<<<nc, RT, 0, ctx.stream>>>(refl_chunks(mp), nb, part, T, ldt, W2);
-    NC_CHECK_LAUNCH();
-    refl_apply_kernel<<<refl_chunks(mp), RT, RA_SMEM, ctx.stream>>>(mp, nb, V, ldv, W2, C, ldc, nc);
-    NC_CHECK_LAUNCH();
-    ctx.launches += 2;
+// Q <- I - Q (m x n)
+__global__ void one_minus_kernel(long long m, int n, cplx* __restrict__ Q) {
+    const long long total = m * n;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
+         e += (long long)gridDim.x * blockDim.x) {
+        const cplx q = Q[e];
+        Q[e] = cmake((e % m == e / m ? 1.0 : 0.0) - q.x, -q.y);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -821,14 +714,23 @@ void householder_qr(Context& ctx, int m, int n, cplx* A, cplx* Q, cplx* R, bool 
 }
 
 // Look-ahead form of householder_qr for the gauge moves (cluster path only).
-// The main stream (ctx) runs the critical path: factor block k, build T_k,
-// then apply reflector k to block k+1 only, so that block k+1 can be
-// factorised next.  The side stream applies reflector k to the remaining
-// columns and accumulates Q forwards, Q <- Q (I - V_k T_k V_k^H) on an m x m
-// Q, while the main stream factors the following blocks on the cluster's
-// 16 SMs.  Forward accumulation costs about twice the flops of the backward
-// order but overlaps the panels instead of following them.  ev: 2 + 2*nblocks
-// events (fork, join, then per block: T_k ready, bulk update k done).
+// The main stream (ctx) runs the critical path: factor block k, then apply its
+// reflector to block k+1 only, so that block k+1 can be factorised next: one
+// batched product [V^H V, V^H A_{k+1}], a forward substitution in place of T
+// (reflector_solve_kernel) and one rank-64 update.  Beside it the second stream
+// builds T_k, applies the reflector to the remaining columns and extends the
+// compact-WY factor of all reflectors so far,
+//   T <- [T, -T (V^H V_k) T_k; 0, T_k],
+// so that Q needs no pass per block: once the last block is done,
+// Q(:, :n) = I - V (T V_1^H) (V_1 the top n rows of V) is two large products,
+// through residues where those pay.
+// On a B200 a chi = 1024 move (2048 x 1024) goes from 6.23 to 5.04 ms: per
+// block the products between the panels took 130 us on the main stream (partial
+// sums of V^H V and V^H A, T, W2, update), and accumulating Q
+// forwards block by block kept the second stream busy for longer than the
+// panels.
+// ev: 2 + 2*nblocks events (fork, join, then per block: G ready, bulk update
+// done).
 void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int m, int n, cplx* A, cplx* Q,
                               cplx* R, bool conjR) {
     NC_ARG(m >= n && n >= 1 && m <= CQ_MAXC * CQ_MAXR, "householder_qr: need 1 <= n <= m <= 2048");
@@ -838,62 +740,78 @@ void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int 
     const int nblocks = (n + NB - 1) / NB;
     cplx* V = ar.alloc_n<cplx>((size_t)m * n);
     cplx* tau = ar.alloc_n<cplx>(n);
-    cplx* Tb = ar.alloc_n<cplx>((size_t)nblocks * NB * NB);
-    cplx* Gpart = ar.alloc_n<cplx>((size_t)refl_chunks(m) * NB * NB);
-    cplx* Wpart = ar.alloc_n<cplx>((size_t)refl_chunks(m) * NB * NB);
+    cplx* GW = ar.alloc_n<cplx>((size_t)nblocks * 2 * NB * NB);   // per block: V^H V, V^H A_{k+1}
     cplx* W2m = ar.alloc_n<cplx>(NB * NB);
+    cplx* Tb = ar.alloc_n<cplx>(NB * NB);
     cplx* Ws = ar.alloc_n<cplx>((size_t)NB * n);
     cplx* W2s = ar.alloc_n<cplx>((size_t)NB * n);
-    cplx* QW = ar.alloc_n<cplx>((size_t)m * NB);
-    cplx* QW2 = ar.alloc_n<cplx>((size_t)m * NB);
-    cplx* Qf = ar.alloc_n<cplx>((size_t)m * m);
+    cplx* T = ar.alloc_n<cplx>((size_t)n * n);
+    cplx* Z = ar.alloc_n<cplx>((size_t)n * n);
     const uint64_t side0 = side.launches;
+    NC_SET_SMEM_ONCE(reflector_solve_kernel, TRS_SMEM);
 
     NC_CUDA(cudaEventRecord(ev[0], ctx.stream));   // fork
     NC_CUDA(cudaStreamWaitEvent(side.stream, ev[0], 0));
-    identity_cols<<<gsz((long long)m * m), 256, 0, side.stream>>>(m, m, Qf);
+    zero_upper_kernel<<<gsz((long long)n * n), 256, 0, side.stream>>>(n, V, m, T);
     NC_CHECK_LAUNCH();
     side.launches++;
     for (int ob = 0; ob < nblocks; ++ob) {
         const int j0 = ob * NB, nb = std::min(NB, n - j0), mp = m - j0;
-        const cplx* Vb = V + j0 + j0 * (long long)m;
-        cplx* T = Tb + (size_t)ob * NB * NB;
-        cudaEvent_t ev_t = ev[2 + 2 * ob], ev_bulk = ev[3 + 2 * ob];
-        // main: factor block ob, then T_ob from the chunk partials of V^H V
-        launch_cluster_block(ctx, mp, nb, A + j0 + j0 * lda, lda, V + j0 + j0 * (long long)m, m, tau + j0);
-        launch_refl_partial(ctx, mp, nb, Vb, m, Vb, m, nb, Gpart);
-        launch_build_t(ctx, nb, Gpart, tau + j0, T, refl_chunks(mp));
-        NC_CUDA(cudaEventRecord(ev_t, ctx.stream));
         const int j1 = j0 + nb, nb1 = (ob + 1 < nblocks) ? std::min(NB, n - j1) : 0;
-        if (nb1 > 0) {
-            // main: reflector ob on block ob+1, after the side stream's update of
-            // those columns by reflector ob-1
-            if (ob > 0) NC_CUDA(cudaStreamWaitEvent(ctx.stream, ev[3 + 2 * (ob - 1)], 0));
-            cplx* A1 = A + j0 + j1 * lda;
-            launch_refl_partial(ctx, mp, nb, Vb, m, A1, lda, nb1, Wpart);
-            launch_refl_finish(ctx, mp, nb, Vb, m, T, NB, Wpart, W2m, A1, lda, nb1);
+        const cplx* Vb = V + j0 + j0 * (long long)m;
+        cplx* G = GW + (size_t)ob * 2 * NB * NB;
+        cplx* W = G + NB * NB;
+        cplx* A1 = A + j0 + j1 * lda;
+        cudaEvent_t ev_g = ev[2 + 2 * ob], ev_bulk = ev[3 + 2 * ob];
+        // main: factor block ob; its reflector on block ob+1, after the second
+        // stream's update of those columns by reflector ob-1
+        launch_cluster_block(ctx, mp, nb, A + j0 + j0 * lda, lda, V + j0 + j0 * (long long)m, m, tau + j0);
+        if (nb1 > 0 && ob > 0) NC_CUDA(cudaStreamWaitEvent(ctx.stream, ev[3 + 2 * (ob - 1)], 0));
+        ZGemmParams g = zgemm_params(OP_C, OP_N, nb, nb, mp, Vb, m, Vb, m, G, nb);
+        if (nb1 == nb) {   // both products as one batch: A and V have the same leading dimension
+            g.batch = 2;
+            g.sB0 = A1 - Vb;
+            g.sC0 = NB * NB;
         }
-        // side: reflector ob on the columns after block ob+1, then Q
-        NC_CUDA(cudaStreamWaitEvent(side.stream, ev_t, 0));
+        zgemm(g, ctx);
+        if (nb1 > 0 && nb1 != nb) zgemm(zgemm_params(OP_C, OP_N, nb, nb1, mp, Vb, m, A1, lda, W, nb), ctx);
+        NC_CUDA(cudaEventRecord(ev_g, ctx.stream));
+        if (nb1 > 0) {
+            reflector_solve_kernel<<<ceil_div(nb1, TRS_WARPS), 32 * TRS_WARPS, TRS_SMEM, ctx.stream>>>(nb, nb1, G, tau + j0,
+                                                                                                      W, W2m);
+            NC_CHECK_LAUNCH();
+            ctx.launches++;
+            ZGemmParams u = zgemm_params(OP_N, OP_N, mp, nb1, nb, Vb, m, W2m, nb, A1, lda);
+            u.alpha = cmake(-1, 0);
+            u.beta = cmake(1, 0);
+            zgemm(u, ctx);
+        }
+        // side: T_ob, the reflector on the columns after block ob+1, the full T
+        NC_CUDA(cudaStreamWaitEvent(side.stream, ev_g, 0));
+        launch_build_t(side, nb, G, tau + j0, Tb);
         const int jr = j1 + nb1, nt = n - jr;
         if (nt > 0) {
             cplx* A2 = A + j0 + jr * lda;
             zgemm(zgemm_params(OP_C, OP_N, nb, nt, mp, Vb, m, A2, lda, Ws, nb), side);
-            zgemm(zgemm_params(OP_C, OP_N, nb, nt, nb, T, NB, Ws, nb, W2s, nb), side);
+            zgemm(zgemm_params(OP_C, OP_N, nb, nt, nb, Tb, NB, Ws, nb, W2s, nb), side);
             ZGemmParams p = zgemm_params(OP_N, OP_N, mp, nt, nb, Vb, m, W2s, nb, A2, lda);
             p.alpha = cmake(-1, 0);
             p.beta = cmake(1, 0);
             zgemm(p, side);
         }
         NC_CUDA(cudaEventRecord(ev_bulk, side.stream));
-        // Qf(:, j0:) -= (Qf(:, j0:) V_ob) T_ob V_ob^H
-        cplx* Qs = Qf + j0 * (long long)m;
-        zgemm(zgemm_params(OP_N, OP_N, m, nb, mp, Qs, m, Vb, m, QW, m), side);
-        zgemm(zgemm_params(OP_N, OP_N, m, nb, nb, QW, m, T, NB, QW2, m), side);
-        ZGemmParams q = zgemm_params(OP_N, OP_C, m, mp, nb, QW2, m, Vb, m, Qs, m);
-        q.alpha = cmake(-1, 0);
-        q.beta = cmake(1, 0);
-        zgemm(q, side);
+        if (!Q) continue;
+        place_t_kernel<<<1, 256, 0, side.stream>>>(nb, Tb, T + j0 + j0 * (long long)n, n);
+        NC_CHECK_LAUNCH();
+        side.launches++;
+        if (j0 > 0) {
+            // V(:, :j0)^H V_ob over the rows where V_ob is not zero
+            zgemm(zgemm_params(OP_C, OP_N, j0, nb, mp, V + j0, m, Vb, m, Ws, j0), side);
+            zgemm(zgemm_params(OP_N, OP_N, j0, nb, j0, T, n, Ws, j0, W2s, j0), side);
+            ZGemmParams p = zgemm_params(OP_N, OP_N, j0, nb, nb, W2s, j0, Tb, NB, T + j0 * (long long)n, n);
+            p.alpha = cmake(-1, 0);
+            zgemm(p, side);
+        }
     }
     NC_CUDA(cudaEventRecord(ev[1], side.stream));   // join
     NC_CUDA(cudaStreamWaitEvent(ctx.stream, ev[1], 0));
@@ -903,7 +821,26 @@ void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int 
         NC_CHECK_LAUNCH();
         ctx.launches++;
     }
-    if (Q) NC_CUDA(cudaMemcpyAsync(Q, Qf, sizeof(cplx) * (size_t)m * n, cudaMemcpyDeviceToDevice, ctx.stream));
+    if (!Q) return;
+    // Z = T V_1^H, Q = I - V Z
+    ResMatrix a, b;
+    if (residue_gemm_pays(n, n, n)) {
+        a.X = T; a.rows = n; a.K = n; a.si = 1; a.sk = n; a.I = n;
+        b.X = V; b.rows = n; b.K = n; b.si = 1; b.sk = m; b.I = n; b.conj = 1;
+        residue_product(ctx, a, b, Z, n, 0, n);
+    } else {
+        zgemm(zgemm_params(OP_N, OP_C, n, n, n, T, n, V, m, Z, n), ctx);
+    }
+    if (residue_gemm_pays(m, n, n)) {
+        a.X = V; a.rows = m; a.K = n; a.si = 1; a.sk = m; a.I = m; a.conj = 0;
+        b.X = Z; b.rows = n; b.K = n; b.si = n; b.sk = 1; b.I = n; b.conj = 0;
+        residue_product(ctx, a, b, Q, m, 0, m);
+    } else {
+        zgemm(zgemm_params(OP_N, OP_N, m, n, n, V, m, Z, n, Q, m), ctx);
+    }
+    one_minus_kernel<<<gsz((long long)m * n), 256, 0, ctx.stream>>>(m, n, Q);
+    NC_CHECK_LAUNCH();
+    ctx.launches++;
 }
 
 // ---------------------------------------------------------------------------
