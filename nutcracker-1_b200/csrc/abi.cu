@@ -179,7 +179,7 @@ int nc_profile_query(int kind, uint64_t* launches, double* total_ms, double* tot
 int nc_synchronize(void) {
     NC_ABI_BEGIN
     NC_CUDA(cudaStreamSynchronize(Context::get().stream));
-    residue_check(Context::get());
+    device_check(Context::get());
     NC_ABI_END
     return g_status;
 }

@@ -566,7 +566,7 @@ struct Chain {
             tc_check(ctx);
             stats.mixed_sweeps++;
         }
-        residue_check(ctx);
+        device_check(ctx);
         if (free_sweeps > 0) --free_sweeps;
         stats.sweeps++;
         emit(NC_SIGNAL_SWEEP_PERFORMED, (int64_t)stats.sweeps);   // chain.cpp:162

@@ -45,7 +45,7 @@ struct HostStage {
     }
     void sync() {
         NC_CUDA(cudaStreamSynchronize(ctx.stream));
-        residue_check(ctx);
+        device_check(ctx);
     }
 
     MpoSite mpo(uint32_t d, uint32_t cl, uint32_t cr, uint32_t nnz, const uint32_t* idx,

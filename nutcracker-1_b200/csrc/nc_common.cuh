@@ -98,7 +98,8 @@ struct Context {
     size_t pinned_bytes = 0;
     uint64_t launches = 0;   // kernels launched by this library on this context
     int krylov_dim = 24;     // Lanczos basis size before a restart
-    bool residue_used = false;   // a residue GEMM was launched since the last residue_check
+    // a kernel with bounded waits (residue GEMM, cluster QR) was launched since the last device_check
+    bool check_pending = false;
     // Gauge of the Level-0 norm_denorm_* / norm_for_* entry points: true
     // (default) = the reference's exact polar factor, false = the faster
     // Householder-QR gauge (the same state, a different site tensor).

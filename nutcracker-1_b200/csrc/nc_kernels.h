@@ -146,6 +146,8 @@ int convert_vectors_to_reflectors_dev(Context& ctx, long long m, int n, cplx* A,
 // triangle of A; optional explicit Q (m x n) and R (n x n, zeros below,
 // conjugated if conjR).
 void householder_qr(Context& ctx, int m, int n, cplx* A, cplx* Q, cplx* R, bool conjR);
+// Whether a wait of the cluster QR has expired since the last call (for device_check).
+int qr_take_error();
 
 // ---- tcgen05 3xTF32 complex GEMM (tc32.cu) ---------------------------------
 // One operand of the real GEMM: rows x Kr floats, Kr contiguous, row stride
@@ -189,9 +191,10 @@ bool residue_gemm_pays(long long M, long long N, long long K);
 // from ctx.scratch()).
 void residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b, cplx* C, int I, long long sI,
                      long long sn);
-// Synchronises ctx.stream and raises NC_ERR_TIMEOUT if a wait of a residue
-// GEMM launched since the last check expired; returns at once when none was.
-void residue_check(Context& ctx);
+// Synchronises ctx.stream and raises NC_ERR_TIMEOUT if a bounded wait of a
+// residue GEMM or cluster QR launched since the last check expired; returns at
+// once when none was.
+void device_check(Context& ctx);
 
 // ---- precision form of the site products (mixed.cu) ------------------------
 // Tensor-core operands of one site's H_eff (environments expanded once per

@@ -534,13 +534,346 @@ cluster_block_qr_kernel(int mp, int nb, int rows_per_cta, cplx* __restrict__ A, 
     cluster.sync();   // no CTA leaves while another may still write its shared memory
 }
 
+// ---------------------------------------------------------------------------
+// The same block factorised eight columns at a time, for the shapes of more
+// than one block.
+//
+// What bounds cluster_block_qr_kernel is the chain of one column: partial sums
+// of all trailing columns (FP64 pipe), exchange, reflector, update of all
+// trailing columns (FP64 pipe), 3.3 us of it at 16 CTAs.  Here the chain of a
+// column only involves the eight columns of its sub-block: thread (c, r) holds
+// rows r and r + 64 of column c, two rows instead of sixteen.  The other
+// columns get the eight reflectors at once,
+//   P <- P - V W2,  W2 = T^H (V^H P)  (T 8 x 8, compact WY),
+// on the FP64 tensor pipe (M = 8 reflectors or columns fits its m8n8k4 shape),
+// with V^H P summed over the CTAs by column slices once per sub-block.  v_c^H v_i for i < c
+// comes out of the column's own sums (they run over all eight columns), so it
+// costs nothing.  B200, one 2048 x 64 block: 212 -> SUBUS us.
+//
+// The one-block shapes (n <= 64) keep the kernel above: their results stay what
+// they were bit for bit (a chain's edge sites turn rounding into the phase of
+// the state).
+// ---------------------------------------------------------------------------
+constexpr int SB = 8;             // columns per sub-block
+constexpr int VP = CQ_MAXR + 1;   // pitch of the reflectors: neighbours start in neighbouring banks
+constexpr int RS = 640;           // C x ceil(64 / C) x SB at most, over C = 1 .. 16
+struct SubSmem {
+    cplx recvW[RS];                   // V^H P partial sums of this CTA's columns, by source CTA
+    cplx recv[2][SB][2 * CQ_MAXC];    // column sums by source half CTA, per column parity
+    cplx piv[2][SB];                  // pivot row, per column parity
+    cplx xs[2][CQ_MAXR];              // the column's rows, per parity
+    cplx v[SB][VP];                   // the reflectors, explicit
+    cplx col[SB][CQ_MAXR];            // the columns: R above, beta on and v below the diagonal
+    cplx part[NB][SB];                // V^H P over the second 64 rows; then W2
+    cplx G[SB][SB];                   // G[c][i] = v_c^H v_i, i < c
+    cplx T[SB][SB];                   // compact-WY factor of the sub-block, T[g][i] = conj(T(i, g))
+    cplx tau[SB];
+    cplx taus[NB];
+    unsigned long long bar[2];        // arrival of a column's sums, per parity
+};
+
+// Remote stores whose arrival the receiver waits for on its own mbarrier
+// (st.async): a column needs one way through the cluster, not a cluster barrier
+// with its stores before it (2.9 -> 1.9 thousand cycles a column at 16 CTAs).
+// The wait is bounded by the global timer and reports through g_qr_error.
+__device__ int g_qr_error = 0;
+__device__ __forceinline__ uint32_t remote(const void* p, int cta) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(cta));
+    return r;
+}
+__device__ __forceinline__ void send8(uint32_t to, double v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(to),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ bool arrived(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void wait_sums(uint32_t bar, uint32_t parity, bool& alive) {
+    if (!alive || arrived(bar, parity)) return;
+    unsigned long long t0, t1;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    while (!arrived(bar, parity)) {
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+        if (t1 - t0 > 2000000000ull) {   // give up for good: every later wait returns at once
+            atomicExch(&g_qr_error, 1);
+            alive = false;
+            return;
+        }
+    }
+}
+
+__device__ __forceinline__ void qr_dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// Column g of the sub-block's T by one warp, lane i < SB:
+// T(i,g) = -tau_g sum_{i<=l<g} T(i,l) v_l^H v_g, products first, then a tree.
+__device__ __forceinline__ void t_column(SubSmem& s, int g, int lane) {
+    if (lane >= SB) return;
+    cplx x[SB];
+#pragma unroll
+    for (int l = 0; l < SB - 1; ++l) x[l] = l < g ? cmul(s.T[l][lane], s.G[g][l]) : cmake(0, 0);   // conjugates of both
+    const cplx sum = cadd(cadd(cadd(x[0], x[1]), cadd(x[2], x[3])), cadd(cadd(x[4], x[5]), x[6]));
+    const cplx tg = cconj(s.tau[g]);
+    s.T[g][lane] = lane < g ? cscale(cmul(tg, sum), -1.0) : lane == g ? tg : cmake(0, 0);
+}
+
+__global__ void __launch_bounds__(CQ_T, 1)
+cluster_subblock_qr_kernel(int mp, int nb, int rows_per_cta, cplx* __restrict__ A, long long lda,
+                           cplx* __restrict__ V, long long ldv, cplx* __restrict__ tau_out) {
+    extern __shared__ __align__(16) unsigned char sub_smem[];
+    SubSmem& s = *reinterpret_cast<SubSmem*>(sub_smem);
+    cg::cluster_group cluster = cg::this_cluster();
+    const int C = (int)cluster.num_blocks();
+    const int rank = (int)cluster.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31;
+    // Whole block: warp (ct, h) holds columns 8 ct .. + 7, rows 64 h .. + 63; lane (n, q) column
+    // 8 ct + n, rows 64 h + 8 t + 2 q + e in a[2 t + e].  That is the B operand of an m8n8k4 FP64
+    // MMA with K over four of the rows (V^H P) and the accumulator of one with the columns as
+    // its rows (P^T - W2^T V^T), so both run from registers.
+    const int ct = tid >> 6, h = (tid >> 5) & 1, n = lane >> 2, q4 = lane & 3;
+    const int k = 8 * ct + n, rbase = 64 * h + 2 * q4;
+    const int c = tid >> 6, r0 = tid & 63, r1 = r0 + 64;       // sub-block: column c, rows r0 and r1
+    const int row0 = rank * rows_per_cta;
+    const int nr = max(0, min(rows_per_cta, mp - row0));
+    const bool top = rank == 0;   // holds all pivot rows (rows_per_cta >= 64 whenever C > 1)
+    int span = 2;                 // lanes that hold one column sum's sources: 2 C, rounded up to a power of two
+    while (span < 2 * C) span <<= 1;
+    const int slice = (NB + C - 1) / C;   // columns per CTA of the exchanged V^H P
+    const uint32_t bars = (uint32_t)__cvta_generic_to_shared(s.bar);
+    const uint32_t column_bytes = (uint32_t)C * SB * 2 * 16 + SB * 16;   // sums of C CTAs, the pivot row
+    bool alive = true;
+    if (tid == 0) {
+        for (int b = 0; b < 2; ++b) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * b) : "memory");
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 8 * b), "r"(column_bytes)
+                         : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    static_assert(CQ_T == 64 * SB && CQ_MAXR == 128 && NB == 64, "thread layouts");
+
+    cplx a[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int r = rbase + 8 * (i >> 1) + (i & 1);
+        a[i] = (r < nr && k < nb) ? A[(row0 + r) + (long long)k * lda] : cmake(0, 0);
+    }
+    for (int c0 = 0; c0 < nb; c0 += SB) {
+        const int w = min(SB, nb - c0);
+        const bool owner = 8 * ct == c0;
+        if (owner) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int r = rbase + 8 * (i >> 1) + (i & 1);
+                s.col[n][r] = a[i];
+                if (n == 0) s.xs[0][r] = a[i];
+            }
+        }
+        if (c0 == 0) cluster.sync();   // every CTA runs before the first remote store
+        else __syncthreads();
+        cplx p0 = s.col[c][r0], p1 = s.col[c][r1];
+        for (int jj = 0; jj < w; ++jj) {
+            const int j = c0 + jj, p = jj & 1;
+            // sums below the diagonal of conj(x) times every column of the sub-block
+            const cplx x0 = s.xs[p][r0], x1 = s.xs[p][r1];
+            double sr = 0, si = 0;
+            if (!top || r0 > j) {
+                sr = fma(x0.x, p0.x, x0.y * p0.y);
+                si = fma(x0.x, p0.y, -x0.y * p0.x);
+            }
+            sr = fma(x1.x, p1.x, fma(x1.y, p1.y, sr));   // r1 >= 64 > j
+            si = fma(x1.x, p1.y, fma(-x1.y, p1.x, si));
+            {
+                // lanes 0-15 go on with the real part, 16-31 with the imaginary one
+                const bool up = lane & 16;
+                const double pvx = __shfl_sync(0xffffffffu, p0.x, j & 31), pvy = __shfl_sync(0xffffffffu, p0.y, j & 31);
+                const double pv = up ? pvy : pvx;   // the pivot row, in the warps that hold it
+                double sum = (up ? si : sr) + __shfl_xor_sync(0xffffffffu, up ? sr : si, 16);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                // lane d (and d + 16) to CTA d
+                const int d = lane & 15;
+                if (d < C) {
+                    const uint32_t bar = remote(&s.bar[p], d);
+                    send8(remote(&s.recv[p][c][2 * rank + h], d) + (up ? 8 : 0), sum, bar);
+                    if (top && h == (j >> 5)) send8(remote(&s.piv[p][c], d) + (up ? 8 : 0), pv, bar);
+                }
+            }
+            if (tid < 32 && jj > 0) t_column(s, jj - 1, lane);   // while the sums travel
+            wait_sums(bars + 8 * p, (uint32_t)(j >> 1) & 1u, alive);
+            // every thread: the totals of its column and of column jj, in a fixed tree
+            const int src = lane & (span - 1);
+            cplx Sc = src < 2 * C ? s.recv[p][c][src] : cmake(0, 0);
+            double Sj = src < 2 * C ? s.recv[p][jj][src].x : 0.0;
+            for (int o = span >> 1; o > 0; o >>= 1) {
+                Sc.x += __shfl_xor_sync(0xffffffffu, Sc.x, o);
+                Sc.y += __shfl_xor_sync(0xffffffffu, Sc.y, o);
+                Sj += __shfl_xor_sync(0xffffffffu, Sj, o);
+            }
+            const cplx alpha = s.piv[p][jj], pc = s.piv[p][c];
+            cplx t = cmake(0, 0), scale = cmake(1, 0), diag = alpha;
+            const bool reflect = !(Sj == 0.0 && alpha.y == 0.0);
+            if (reflect) {
+                const double beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + Sj), alpha.x);
+                const cplx den = cmake(alpha.x - beta, alpha.y);
+                const double ib = 1.0 / beta;
+                const double idd = 1.0 / (den.x * den.x + den.y * den.y);
+                t = cmake((beta - alpha.x) * ib, -alpha.y * ib);
+                scale = cmake(den.x * idd, -den.y * idd);
+                diag = cmake(beta, 0);
+            }
+            const bool below0 = !top || r0 > j;
+            const cplx v0 = cmul(x0, scale), v1 = cmul(x1, scale);   // the reflector below its pivot
+            if (c > jj) {
+                if (reflect) {
+                    const cplx cf = cmul(cconj(t), cadd(pc, cmul(cconj(scale), Sc)));
+                    if (below0) p0 = csub(p0, cmul(v0, cf));
+                    else if (r0 == j) p0 = csub(p0, cf);
+                    p1 = csub(p1, cmul(v1, cf));
+                }
+                if (c == jj + 1) {
+                    s.xs[p ^ 1][r0] = p0;
+                    s.xs[p ^ 1][r1] = p1;
+                }
+            } else if (c == jj) {
+                s.v[jj][r0] = below0 ? v0 : cmake(r0 == j ? 1.0 : 0.0, 0.0);
+                s.v[jj][r1] = v1;
+                if (below0) p0 = v0;
+                else if (r0 == j) p0 = diag;
+                p1 = v1;
+                if (r0 == 0) {
+                    s.tau[jj] = t;
+                    s.taus[j] = t;
+                }
+            } else if (r0 == 0) {
+                s.G[jj][c] = cadd(pc, cmul(cconj(scale), Sc));   // v_jj^H v_c, column c holding v_c below its pivot
+            }
+            __syncthreads();
+            // every thread is past its wait: the barrier's next use is armed
+            if (tid == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 8 * p), "r"(column_bytes)
+                             : "memory");
+        }
+        // the finished columns back to their owners: R above, beta on and v below the diagonal
+        s.col[c][r0] = p0;
+        s.col[c][r1] = p1;
+        __syncthreads();
+        if (owner && n < w) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) a[i] = s.col[n][rbase + 8 * (i >> 1) + (i & 1)];
+        }
+        if (c0 + SB >= nb) break;
+        const bool mine = 8 * ct > c0;   // the warp's columns are to the right of the sub-block
+        double wr[2] = {0, 0}, wi[2] = {0, 0};   // (V^H P)(lane / 4, 8 ct + 2 (lane % 4) + {0, 1})
+        if (mine) {
+            double ur[2] = {0, 0}, ui[2] = {0, 0};
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const cplx v = s.v[n][rbase + 8 * (i >> 1) + (i & 1)];   // reflector n, this lane's row
+                qr_dmma(wr, v.x, a[i].x);
+                qr_dmma(ur, v.y, a[i].y);
+                qr_dmma(wi, v.x, a[i].y);
+                qr_dmma(ui, -v.y, a[i].x);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                wr[e] += ur[e];
+                wi[e] += ui[e];
+            }
+            if (h == 1) {
+                s.part[8 * ct + 2 * q4][n] = cmake(wr[0], wi[0]);
+                s.part[8 * ct + 2 * q4 + 1][n] = cmake(wr[1], wi[1]);
+            }
+        } else if (tid < 32) {
+            t_column(s, SB - 1, lane);   // warp 0 never holds columns to the right
+        }
+        __syncthreads();
+        if (mine && h == 0) {
+            // each column's sums go to the CTA that finishes it
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int kk = 8 * ct + 2 * q4 + e;
+                const cplx u = s.part[kk][n];
+                cluster.map_shared_rank(s.recvW, kk / slice)[(rank * slice + kk % slice) * SB + n] =
+                    cmake(wr[e] + u.x, wi[e] + u.y);
+            }
+        }
+        cluster.sync();
+        {
+            // W2 = T^H W, one column per eight lanes, sent to every CTA
+            const int g = tid & 7, first = rank * slice, kk = first + (tid >> 3);
+            const bool on = kk < min(NB, first + slice) && kk >= c0 + SB;
+            cplx W = cmake(0, 0);
+            if (on)
+                for (int d = 0; d < C; ++d) W = cadd(W, s.recvW[(d * slice + kk - first) * SB + g]);
+            cplx x[SB];
+#pragma unroll
+            for (int i = 0; i < SB; ++i) {
+                x[i] = cmake(__shfl_sync(0xffffffffu, W.x, (lane & ~7) | i),
+                             __shfl_sync(0xffffffffu, W.y, (lane & ~7) | i));
+                x[i] = cmul(s.T[g][i], x[i]);   // zero for i > g
+            }
+            const cplx w2 = cadd(cadd(cadd(x[0], x[1]), cadd(x[2], x[3])), cadd(cadd(x[4], x[5]), cadd(x[6], x[7])));
+            if (on)
+                for (int d = 0; d < C; ++d) cluster.map_shared_rank(&s.part[kk][0], d)[g] = w2;
+        }
+        cluster.sync();
+        if (mine) {
+            const cplx w0 = s.part[k][q4], w1 = s.part[k][q4 + 4];
+#pragma unroll
+            for (int t8 = 0; t8 < 8; ++t8) {
+                double cr[2] = {a[2 * t8].x, a[2 * t8 + 1].x}, ci[2] = {a[2 * t8].y, a[2 * t8 + 1].y};
+                const cplx v0 = s.v[q4][64 * h + 8 * t8 + n], v1 = s.v[q4 + 4][64 * h + 8 * t8 + n];
+                qr_dmma(cr, -w0.x, v0.x);
+                qr_dmma(ci, -w0.y, v0.x);
+                qr_dmma(cr, w0.y, v0.y);
+                qr_dmma(ci, -w0.x, v0.y);
+                qr_dmma(cr, -w1.x, v1.x);
+                qr_dmma(ci, -w1.y, v1.x);
+                qr_dmma(cr, w1.y, v1.y);
+                qr_dmma(ci, -w1.x, v1.y);
+                a[2 * t8] = cmake(cr[0], ci[0]);
+                a[2 * t8 + 1] = cmake(cr[1], ci[1]);
+            }
+        }
+        __syncthreads();   // s.v, s.col, s.part are rewritten by the next sub-block
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int r = rbase + 8 * (i >> 1) + (i & 1), prow = row0 + r;
+        if (r < nr && k < nb) {
+            A[prow + (long long)k * lda] = a[i];
+            V[prow + (long long)k * ldv] = (prow > k) ? a[i] : cmake(prow == k ? 1.0 : 0.0, 0);
+        }
+    }
+    if (top)
+        for (int q = tid; q < nb; q += CQ_T) tau_out[q] = s.taus[q];
+    cluster.sync();   // no CTA leaves while another may still write its shared memory
+}
+
 // Cluster launch support (size CQ_MAXC needs the non-portable opt-in); a
 // device that cannot co-schedule the cluster uses the per-panel path.
 // The attribute and the answer belong to each device, so both are kept per
 // device (the first 64; others are probed on every call).
 bool cluster_qr_probe() {
     if (cudaFuncSetAttribute(cluster_block_qr_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-        cudaSuccess) {
+            cudaSuccess ||
+        cudaFuncSetAttribute(cluster_subblock_qr_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(cluster_subblock_qr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(SubSmem)) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -554,13 +887,32 @@ bool cluster_qr_probe() {
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    int nclusters = 0;
+    int nclusters = 0, nsub = 0;
     if (cudaOccupancyMaxActiveClusters(&nclusters, cluster_block_qr_kernel, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return nclusters >= 1;
+    cfg.dynamicSmemBytes = sizeof(SubSmem);
+    if (cudaOccupancyMaxActiveClusters(&nsub, cluster_subblock_qr_kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return nclusters >= 1 && nsub >= 1;
 }
+
+}  // namespace
+
+int qr_take_error() {
+    int flag = 0;
+    NC_CUDA(cudaMemcpyFromSymbol(&flag, g_qr_error, sizeof(int)));
+    if (flag) {
+        const int zero = 0;
+        NC_CUDA(cudaMemcpyToSymbol(g_qr_error, &zero, sizeof(int)));
+    }
+    return flag;
+}
+
+namespace {
 
 bool cluster_qr_available() {
     static std::atomic<int> state[64];   // 0 unknown, 1 available, 2 not available
@@ -575,7 +927,8 @@ bool cluster_qr_available() {
     return s == 1;
 }
 
-void launch_cluster_block(Context& ctx, int mp, int nb, cplx* A, long long lda, cplx* V, long long ldv,
+// `sub`: eight columns at a time (the shapes of several blocks).
+void launch_cluster_block(Context& ctx, bool sub, int mp, int nb, cplx* A, long long lda, cplx* V, long long ldv,
                           cplx* tau) {
     const int C = std::max(1, std::min(CQ_MAXC, (mp + CQ_MAXR - 1) / CQ_MAXR));
     const int rows = (mp + C - 1) / C;
@@ -590,7 +943,13 @@ void launch_cluster_block(Context& ctx, int mp, int nb, cplx* A, long long lda, 
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    NC_CUDA(cudaLaunchKernelEx(&cfg, cluster_block_qr_kernel, mp, nb, rows, A, lda, V, ldv, tau));
+    if (sub) {
+        cfg.dynamicSmemBytes = sizeof(SubSmem);
+        NC_CUDA(cudaLaunchKernelEx(&cfg, cluster_subblock_qr_kernel, mp, nb, rows, A, lda, V, ldv, tau));
+        ctx.check_pending = true;
+    } else {
+        NC_CUDA(cudaLaunchKernelEx(&cfg, cluster_block_qr_kernel, mp, nb, rows, A, lda, V, ldv, tau));
+    }
     ctx.launches++;
 }
 
@@ -654,7 +1013,7 @@ void householder_qr(Context& ctx, int m, int n, cplx* A, cplx* Q, cplx* R, bool 
         const cplx* Vb = V + j0 + j0 * (long long)m;
         cplx* T = Tb + (size_t)ob * NB * NB;
         if (use_cluster) {
-            launch_cluster_block(ctx, mp, nb, A + j0 + j0 * lda, lda, V + j0 + j0 * (long long)m, m, tau + j0);
+            launch_cluster_block(ctx, n > NB, mp, nb, A + j0 + j0 * lda, lda, V + j0 + j0 * (long long)m, m, tau + j0);
             zgemm(zgemm_params(OP_C, OP_N, nb, nb, mp, Vb, m, Vb, m, G, nb), ctx);
         } else {
             for (int jj = j0; jj < j0 + nb; jj += JB) {
@@ -724,11 +1083,11 @@ void householder_qr(Context& ctx, int m, int n, cplx* A, cplx* Q, cplx* R, bool 
 // so that Q needs no pass per block: once the last block is done,
 // Q(:, :n) = I - V (T V_1^H) (V_1 the top n rows of V) is two large products,
 // through residues where those pay.
-// On a B200 a chi = 1024 move (2048 x 1024) goes from 6.23 to 5.04 ms: per
-// block the products between the panels took 130 us on the main stream (partial
-// sums of V^H V and V^H A, T, W2, update), and accumulating Q
-// forwards block by block kept the second stream busy for longer than the
-// panels.
+// On a B200 a chi = 1024 move (2048 x 1024) goes from 6.23 to 3.75 ms (with the
+// panels of cluster_subblock_qr_kernel): per block the products between the
+// panels took 130 us on the main stream (partial sums of V^H V and V^H A, T, W2,
+// update), and accumulating Q forwards block by block kept the second stream
+// busy for longer than the panels.
 // ev: 2 + 2*nblocks events (fork, join, then per block: G ready, bulk update
 // done).
 void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int m, int n, cplx* A, cplx* Q,
@@ -765,7 +1124,7 @@ void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int 
         cudaEvent_t ev_g = ev[2 + 2 * ob], ev_bulk = ev[3 + 2 * ob];
         // main: factor block ob; its reflector on block ob+1, after the second
         // stream's update of those columns by reflector ob-1
-        launch_cluster_block(ctx, mp, nb, A + j0 + j0 * lda, lda, V + j0 + j0 * (long long)m, m, tau + j0);
+        launch_cluster_block(ctx, true, mp, nb, A + j0 + j0 * lda, lda, V + j0 + j0 * (long long)m, m, tau + j0);
         if (nb1 > 0 && ob > 0) NC_CUDA(cudaStreamWaitEvent(ctx.stream, ev[3 + 2 * (ob - 1)], 0));
         ZGemmParams g = zgemm_params(OP_C, OP_N, nb, nb, mp, Vb, m, Vb, m, G, nb);
         if (nb1 == nb) {   // both products as one batch: A and V have the same leading dimension
@@ -926,6 +1285,7 @@ cudaStream_t priority_stream() {
 // Run the QR of plan.X; the first run of a shape executes directly (so the
 // private arena grows to its final size) and then records the graph.
 void qr_run(Context& ctx, QrPlan& P) {
+    if (P.lookahead && P.capture) ctx.check_pending = true;
     if (P.exec) {
         NC_CUDA(cudaGraphLaunch(P.exec, ctx.stream));
         ctx.launches += P.kernels;
@@ -994,8 +1354,17 @@ void qr_run(Context& ctx, QrPlan& P) {
 }  // namespace
 
 // The absorption GEMM of the gauge factor, on ctx.stream or, with `as`, on
-// the second stream after the QR that produced the factor.
-static void absorb_factor(Context& ctx, const ZGemmParams& p, const AbsorbAsync* as) {
+// the second stream after the QR that produced the factor.  A product that pays
+// through residues (a, b: the same one) runs on ctx.stream in either case: it
+// needs the context's scratch, and it is shorter than what it would hide behind
+// (chi = 1024: 605 us on the FP64 pipe, 160 through residues, B200).
+static void absorb_factor(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResMatrix& b, int I,
+                          long long sI, long long sn, const AbsorbAsync* as) {
+    if (residue_gemm_pays(a.rows, b.rows, a.K)) {
+        residue_product(ctx, a, b, p.C, I, sI, sn);
+        if (as) NC_CUDA(cudaEventRecord(as->done, ctx.stream));
+        return;
+    }
     if (!as) {
         zgemm(p, ctx);
         return;
@@ -1020,7 +1389,10 @@ void gauge_right(Context& ctx, int bl, int bm, int br, int dl, int dr, const cpl
         ZGemmParams p = zgemm_params(OP_N, OP_C, br, bm, bm, B, br, P.R, bm, denormB, br);
         p.batch = dr;
         p.sA0 = (long long)br * bm; p.sB0 = 0; p.sC0 = (long long)br * bm;
-        absorb_factor(ctx, p, async);
+        ResMatrix a, b;   // rows (r, s) of B against the rows of conj(Rt)
+        a.X = B; a.rows = br * dr; a.K = bm; a.si = 1; a.I = br; a.sI = (long long)br * bm; a.sk = br;
+        b.X = P.R; b.rows = bm; b.K = bm; b.si = 1; b.I = bm; b.sk = bm; b.conj = 1;
+        absorb_factor(ctx, p, a, b, br, (long long)br * bm, br, async);
     }
     permute3(ctx, P.Q, K, bm, 1, p_t, true, normA);         // normA = Qt^H
 }
@@ -1036,7 +1408,10 @@ void gauge_left(Context& ctx, int bl, int bm, int br, int dl, int dr, const cplx
     qr_run(ctx, P);                                          // Rc = conj(Rt)
     if (A && denormA) {
         // denormA = conj(Rt) * A  (as bm x bl*dl)
-        absorb_factor(ctx, zgemm_params(OP_N, OP_N, bm, bl * dl, bm, Rc, bm, A, bm, denormA, bm), async);
+        ResMatrix a, b;
+        a.X = Rc; a.rows = bm; a.K = bm; a.si = 1; a.I = bm; a.sk = bm;
+        b.X = A; b.rows = bl * dl; b.K = bm; b.si = bm; b.I = b.rows; b.sk = 1;
+        absorb_factor(ctx, zgemm_params(OP_N, OP_N, bm, bl * dl, bm, Rc, bm, A, bm, denormA, bm), a, b, bm, 0, bm, async);
     }
     permute3(ctx, P.Q, br, dr, bm, p_rs, true, normB);       // normB(r,m,s) = conj(Qt((r,s),m))
 }

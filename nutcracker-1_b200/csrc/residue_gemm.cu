@@ -643,7 +643,7 @@ void residue_gemm(Context& ctx, const ResOperand& A, const ResOperand& B, cplx* 
     res_crt_kernel<<<dim3((P.M + 127) / 128, groups), 128, 0, ctx.stream>>>(P.res, o);
     NC_CHECK_LAUNCH();
     ctx.launches += 2;
-    ctx.residue_used = true;
+    ctx.check_pending = true;
 }
 
 }  // namespace
@@ -660,17 +660,19 @@ void residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b, cplx*
     });
 }
 
-void residue_check(Context& ctx) {
-    if (!ctx.residue_used) return;
-    ctx.residue_used = false;
+void device_check(Context& ctx) {
+    if (!ctx.check_pending) return;
+    ctx.check_pending = false;
     NC_CUDA(cudaStreamSynchronize(ctx.stream));
     int flag = 0;
     NC_CUDA(cudaMemcpyFromSymbol(&flag, g_res_error, sizeof(int)));
     if (flag) {
         const int zero = 0;
         NC_CUDA(cudaMemcpyToSymbol(g_res_error, &zero, sizeof(int)));
-        throw Error(NC_ERR_TIMEOUT, "residue GEMM: a pipeline wait exceeded its time limit");
     }
+    const int qr = qr_take_error();
+    if (flag) throw Error(NC_ERR_TIMEOUT, "residue GEMM: a pipeline wait exceeded its time limit");
+    if (qr) throw Error(NC_ERR_TIMEOUT, "cluster QR: an exchange between CTAs exceeded its time limit");
 }
 
 }  // namespace nc
