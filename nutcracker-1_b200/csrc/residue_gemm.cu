@@ -103,7 +103,8 @@ constexpr Tables make_tables() {
     }
     return t;
 }
-__constant__ Tables kT = make_tables();
+constexpr Tables kC = make_tables();
+__constant__ Tables kT = make_tables();   // for a modulus known at run time only
 constexpr double kPh = hi_part(mod_product()), kPl = lo_part(mod_product());
 constexpr int kBadExp = 1 << 30;         // exponent of a row with a non-finite element
 constexpr int kMaxK = 16000;             // |Re|, |Im| sums of K residue products fit in int32
@@ -147,10 +148,10 @@ struct ResPair {
 __global__ void __launch_bounds__(NT) res_norm_kernel(ResPair P) {
     __shared__ double2 red[NT];
     const int w2 = (int)blockIdx.x >= P.nb[0] ? 1 : 0, bx = blockIdx.x - (w2 ? P.nb[0] : 0);
-    const ResSource& s = P.s[w2];
-    if ((int)blockIdx.y >= P.nchunk[w2]) return;
-    double2* part = P.part[w2];
-    const int k0 = blockIdx.y * P.chunk[w2], k1 = min(s.K, k0 + P.chunk[w2]);
+    const ResSource s = w2 ? P.s[1] : P.s[0];
+    if ((int)blockIdx.y >= (w2 ? P.nchunk[1] : P.nchunk[0])) return;
+    double2* part = w2 ? P.part[1] : P.part[0];
+    const int chunk = w2 ? P.chunk[1] : P.chunk[0], k0 = blockIdx.y * chunk, k1 = min(s.K, k0 + chunk);
     double sum = 0, mx = 0;
     auto take = [&](const cplx v) {
         sum = fma(v.x, v.x, fma(v.y, v.y, sum));     // a NaN survives here, fmax drops it
@@ -158,6 +159,7 @@ __global__ void __launch_bounds__(NT) res_norm_kernel(ResPair P) {
     };
     if (s.sk == 1) {
         const cplx* x = row_ptr(s, bx);
+#pragma unroll 4
         for (int k = k0 + threadIdx.x; k < k1; k += NT) take(x[k]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -221,10 +223,14 @@ __device__ __forceinline__ int row_exponent(const double2* __restrict__ part, in
 // elements (the operands of a chi=1024 Heisenberg product) write 1 GB, 0.16 ms
 // at the HBM rate, and cost 15 x 13 integer instructions each.  A residue of
 // the 60-bit integer is two dot products of its bytes with the powers of 2^8
-// modulo p (dp4a), one high multiplication by 2^32 / p and one multiply-add.
-// A thread makes four consecutive K of a row at a time, so that a warp writes
-// a whole 128-byte line of each plane.  A grid too small for the chip is split
-// over the moduli as well.
+// modulo p (dp4a), a quotient rounded in FP32 and one multiply-add.  A thread
+// makes four consecutive K of a row at a time, so that a warp writes a whole
+// 128-byte line of each plane.  The moduli are unrolled, so that their constants
+// are immediates: read from constant memory in a loop they kept the address
+// unit the busiest one, and with the row pointers made once per block instead
+// of per element a chi=768 pair of operands takes 72 us, before 91 (the whole
+// chi=1024 product 1365 us, before 1438).  A grid too small for the chip is
+// split over the moduli as well.
 constexpr int CR = 16, CK = 128;
 // kMagicI (1 - p) + the residue, which is in [0, p): t = 2^8 powers modulo p
 // times the bytes, as the bits of a float; q = round((t - p/2) / p).
@@ -238,11 +244,38 @@ __device__ __forceinline__ uint2 biased(double x, double scale) {
     const unsigned long long v = (unsigned long long)(__double2ll_rn(x * scale) + (1ll << kBias));
     return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
 }
+// The moduli L .. of [l0, l1) for four K of a row; their constants are immediates.
+template <int L>
+__device__ __forceinline__ void residues_of(const uint2 (&vr)[4], const uint2 (&vi)[4], uint8_t*& out, size_t plane, int l0,
+                                            int l1) {
+    if constexpr (L < NL) {
+        if (L >= l0 && L < l1) {
+            constexpr uint32_t p = kC.p[L], m0 = kC.m0[L], m1 = kC.m1[L], off = kC.off[L];
+            constexpr float inv = kC.invf[L], half = kC.half[L];
+            constexpr uint32_t twice = 2 * (kMagicI * (p - 1));
+            uint32_t a[4], b[4], c[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                a[q] = residue(vr[q], m0, m1, off, inv, half, p);
+                b[q] = residue(vi[q], m0, m1, off, inv, half, p);
+                const uint32_t sum = a[q] + b[q] + twice;
+                c[q] = min(sum, sum - p);   // the wrapped difference is large when sum < p
+            }
+            *reinterpret_cast<uint32_t*>(out) = pack4(a[0], a[1], a[2], a[3]);
+            *reinterpret_cast<uint32_t*>(out + plane) = pack4(b[0], b[1], b[2], b[3]);
+            *reinterpret_cast<uint32_t*>(out + 2 * plane) = pack4(c[0], c[1], c[2], c[3]);
+            out += 3 * plane;
+        }
+        residues_of<L + 1>(vr, vi, out, plane, l0, l1);
+    }
+}
+
 __global__ void __launch_bounds__(NT, 4) res_convert_kernel(ResPair P) {
     __shared__ cplx tile[CR][CK + 1];
     __shared__ double scale[CR];
+    __shared__ const cplx* rows[CR];
     const int w2 = (int)blockIdx.x >= P.nb[0] ? 1 : 0, bx = blockIdx.x - (w2 ? P.nb[0] : 0);
-    const ResSource& s = P.s[w2];
+    const ResSource s = w2 ? P.s[1] : P.s[0];
     const int kb = (P.Kp + CK - 1) / CK;
     const int r0 = (bx / kb) * CR, k0 = (bx % kb) * CK;
     const int tid = threadIdx.x;
@@ -250,15 +283,29 @@ __global__ void __launch_bounds__(NT, 4) res_convert_kernel(ResPair P) {
         const int row = r0 + tid;
         int e = 0;
         if (row < s.rows) {
-            e = row_exponent(P.part[w2], P.nchunk[w2], s.rows, row, s.K);
-            if (k0 == 0 && blockIdx.y == 0) P.exps[w2][row] = e;
+            e = row_exponent(w2 ? P.part[1] : P.part[0], w2 ? P.nchunk[1] : P.nchunk[0], s.rows, row, s.K);
+            if (k0 == 0 && blockIdx.y == 0) (w2 ? P.exps[1] : P.exps[0])[row] = e;
         }
         scale[tid] = (e == kBadExp) ? 0.0 : scalbn(1.0, e);
+    } else if (tid >= 32 && tid < 32 + CR) {
+        const int row = r0 + tid - 32;
+        rows[tid - 32] = row < s.rows ? row_ptr(s, row) : nullptr;
     }
-    for (int e = tid; e < CR * CK; e += NT) {
-        const int r = (s.sk == 1) ? e / CK : e % CR, k = (s.sk == 1) ? e % CK : e / CR;
-        const int row = r0 + r, kk = k0 + k;
-        tile[r][k] = (row < s.rows && kk < s.K) ? row_ptr(s, row)[(long long)kk * s.sk] : cmake(0, 0);
+    __syncthreads();
+    if (s.sk == 1) {
+#pragma unroll
+        for (int i = 0; i < CR * CK / NT; ++i) {
+            const int e = tid + i * NT, r = e / CK, k = e % CK;
+            const cplx* x = rows[r];
+            tile[r][k] = (x && k0 + k < s.K) ? x[k0 + k] : cmake(0, 0);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < CR * CK / NT; ++i) {
+            const int e = tid + i * NT, r = e % CR, k = e / CR;
+            const cplx* x = rows[r];
+            tile[r][k] = (x && k0 + k < s.K) ? x[(k0 + k) * s.sk] : cmake(0, 0);
+        }
     }
     __syncthreads();
     const size_t plane = (size_t)s.rows * P.Kp;
@@ -275,24 +322,8 @@ __global__ void __launch_bounds__(NT, 4) res_convert_kernel(ResPair P) {
             vr[q] = biased(v.x, sc);
             vi[q] = biased(s.conj ? -v.y : v.y, sc);
         }
-        uint8_t* out = P.planes[w2] + (size_t)row * P.Kp + k0 + k + (size_t)(3 * l0) * plane;
-#pragma unroll 3
-        for (int l = l0; l < l1; ++l, out += 3 * plane) {
-            const uint32_t p = kT.p[l], m0 = kT.m0[l], m1 = kT.m1[l], off = kT.off[l];
-            const float inv = kT.invf[l], half = kT.half[l];
-            const uint32_t twice = 2 * (kMagicI * (p - 1));
-            uint32_t a[4], b[4], c[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                a[q] = residue(vr[q], m0, m1, off, inv, half, p);
-                b[q] = residue(vi[q], m0, m1, off, inv, half, p);
-                const uint32_t sum = a[q] + b[q] + twice;
-                c[q] = min(sum, sum - p);   // the wrapped difference is large when sum < p
-            }
-            *reinterpret_cast<uint32_t*>(out) = pack4(a[0], a[1], a[2], a[3]);
-            *reinterpret_cast<uint32_t*>(out + plane) = pack4(b[0], b[1], b[2], b[3]);
-            *reinterpret_cast<uint32_t*>(out + 2 * plane) = pack4(c[0], c[1], c[2], c[3]);
-        }
+        uint8_t* out = (w2 ? P.planes[1] : P.planes[0]) + (size_t)row * P.Kp + k0 + k + (size_t)(3 * l0) * plane;
+        residues_of<0>(vr, vi, out, plane, l0, l1);
     }
 }
 
@@ -562,7 +593,7 @@ CUtensorMap make_map8(const uint8_t* ptr, int Kp, int rows, int rows_p, int box_
 
 // Measured on a B200, one H_eff product of a Heisenberg site (two GEMMs and
 // the mix), DMMA route against this one: chi = 192 80 / 116 us, 224 109 / 129,
-// 256 200 / 142, 320 352 / 182, 512 1020 / 369, 1024 5750 / 1440.  The
+// 256 200 / 135, 320 352 / 173, 512 1020 / 345, 1024 5750 / 1362.  The
 // crossing lies near 2^27 complex multiplications a GEMM; below one tile of
 // rows or half a tile of columns the padding costs more.  Error against
 // extended precision (2-norm, chi = 256 / 1024): DMMA 4.3e-16 / 2.2e-15, this
