@@ -14,14 +14,14 @@
 //                        the autotuned table (stage, chi, D, d)
 //   grouped_mix_kernel   the sparse-MPO mix of every chain's site
 //   lz_*_kernel          Lanczos steps: CGS2 reorthogonalisation over
-//                        per-chain vector chunks, then one thread per chain
-//                        for the tridiagonal Ritz problem and the decision
+//                        per-chain vector chunks, then one block per chain
+//                        for the projected problem and the decision
 //   batched_qr_kernel    one CTA per moving chain: Householder QR of the
 //                        site matrix, explicit Q, R for the neighbour
 //
-// A Lanczos iteration (three contraction stages plus eight vector and
-// decision kernels) is captured once as a CUDA graph and replayed: the work
-// lists live in fixed device buffers whose lengths are read on the device.
+// A Lanczos iteration (three contraction stages plus six vector and decision
+// kernels) is captured once as a CUDA graph and replayed: the work lists live
+// in fixed device buffers whose lengths are read on the device.
 //
 // Precision: the batched workload's complex64 products (prec 1: the
 // contractions in complex FP32, the Krylov basis, its reorthogonalisation,
@@ -65,7 +65,6 @@ struct LzChain {
     cplx* V;      // (kMaxKrylov + 1) vectors of length n
     cplx* w;      // residual / scratch vector
     cplx* x;      // the site: initial guess, and the result when accepted
-    cplx* Y;      // (kKeepMax + 1) vectors: the kept Ritz vectors and the residual at a restart
     long long n;
     double tol;
     int cstart, ccount;   // the chain's chunks in the chunk list
@@ -78,7 +77,9 @@ struct LzState {
     int j;          // index of the vector being expanded
     int done;       // 1: converged, failed or not solving this step
     int stall;      // 1: basis full, waiting for a restart
-    int adv;        // 1: the next basis vector is to be written
+    int adv;        // 1: the basis grew by one vector
+    int mv;         // 1: the operator is to be applied to vector jv
+    int jv;
     int restarts, matvecs, fail, accept;
     int fin;        // 1: the solve's result has been taken (or there is no solve)
     double theta, res, beta, tnorm, xnorm, energy;
@@ -275,9 +276,9 @@ __device__ __forceinline__ void gemm_phase(const GProb* __restrict__ probs, cons
             s_local = t - prefix[p];
         }
         __syncthreads();
-        if (st && (st[P.chain].done || st[P.chain].stall)) continue;
+        if (st && !st[P.chain].mv) continue;
         const cplx* A = P.A;
-        if (P.use_jsel) A += (long long)st[P.chain].j * P.a_jstride;
+        if (P.use_jsel) A += (long long)st[P.chain].jv * P.a_jstride;
         const int tm = s_local / P.tiles_n, tn = s_local % P.tiles_n;
         if (P.prec) gemm_dispatch<float>(P, A, tm, tn, smem);
         else gemm_dispatch<double>(P, A, tm, tn, smem);
@@ -312,7 +313,7 @@ __device__ __forceinline__ void mix_phase(const MixProb* __restrict__ probs, con
             s_item = it.y;
         }
         __syncthreads();
-        if (st && (st[P.chain].done || st[P.chain].stall)) continue;
+        if (st && !st[P.chain].mv) continue;
         const int d = P.d, nnz = P.nnz;
         for (int i = threadIdx.x; i < nnz * d * d; i += blockDim.x) Ws[i] = P.W[i];
         for (int i = threadIdx.x; i < nnz; i += blockDim.x) {
@@ -413,115 +414,161 @@ __device__ __forceinline__ void block_sum_c(double (&ar)[NK], double (&ai)[NK], 
     __syncthreads();
 }
 
-// PASS 0: part = V^H w;  PASS 1: w -= V h1, part = V^H w;  PASS 2: w -= V h2, part[0] = |w|^2.
-// Each thread keeps its (at most kVecChunk / kLzT) elements of w in
-// registers; the dot products run four basis vectors at a time, so that every
-// thread has many independent loads in flight, each a fixed-order sum over
-// the chunk.
+// True in the block that is the last of its chain's `count` blocks to arrive
+// (every thread gets the answer); what the others stored before is visible to
+// it.  The counter is back at zero afterwards.
+__device__ __forceinline__ bool last_of_chain(int count, int* counter) {
+    __shared__ int last;
+    if (count == 1) {
+        __syncthreads();
+        return true;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(counter, 1) == count - 1;
+        if (last) *counter = 0;
+    }
+    __syncthreads();
+    __threadfence();
+    return last;
+}
+
+// Warp sums of 8 values, v[i] over the lanes: value i ends in the lanes whose
+// top three bits are i.  Same additions as eight shuffle trees (offsets 16 to
+// 1), 9 shuffles instead of 40: the lanes that would repeat another's sum take
+// over another value instead.
+__device__ __forceinline__ double warp_sum8(const double (&v)[8], int lane) {
+    double a[4], b[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double keep = (lane & 16) ? v[i + 4] : v[i], give = (lane & 16) ? v[i] : v[i + 4];
+        a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const double keep = (lane & 8) ? a[i + 2] : a[i], give = (lane & 8) ? a[i] : a[i + 2];
+        b[i] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+    }
+    const double keep = (lane & 4) ? b[1] : b[0], give = (lane & 4) ? b[0] : b[1];
+    double x = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+    x += __shfl_xor_sync(0xffffffffu, x, 2);
+    x += __shfl_xor_sync(0xffffffffu, x, 1);
+    return x;
+}
+
+// PASS 0: h1 = V^H w;  PASS 1: w -= V h1, h2 = V^H w;  PASS 2: w -= V h2, wn2 = |w|^2.
+// Each thread keeps its (at most kVecChunk / kLzT) elements of w in registers.
+// Chunk sums are stored and added in chunk order by the chain's last chunk, so
+// that the result does not depend on which one that is.  A short chain is bound
+// by latency: the basis is loaded four vectors at a time ahead of the updates
+// and sums that use them, and a block meets once for all its sums.  B200, 12
+// chains of up to 512 elements: 14.5, 16.9 and 13 us for the passes and 4 us
+// for the sum after each, now 12.8, 14.7 and 9.2 us with the sums (from a cold
+// L2, as in the first figures).
 constexpr int kEpt = kVecChunk / kLzT;
 template <int PASS>
-__device__ __forceinline__ void cgs_phase(const VChunk* __restrict__ chunks, const int* __restrict__ nchunks,
-                                          const LzChain* __restrict__ ch, LzState* __restrict__ st,
-                                          cplx* __restrict__ part, int vb, int nvb) {
-    __shared__ cplx red[kLzW * (kMaxKrylov + 1)];
+__global__ void __launch_bounds__(kLzT) lz_cgs_kernel(const VChunk* __restrict__ chunks, const int* __restrict__ nchunks,
+                                                      const LzChain* __restrict__ ch, LzState* __restrict__ st,
+                                                      cplx* __restrict__ part, int* __restrict__ counters) {
+    __shared__ double red[kLzW][2 * (kMaxKrylov + 4)];
     __shared__ cplx hs[kMaxKrylov + 1];
-    const int total = *nchunks;
-    for (int t = vb; t < total; t += nvb) {
+    const int total = *nchunks, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
         const VChunk c = chunks[t];
-        const LzState& S = st[c.chain];
-        if (S.done || S.stall) continue;
+        LzState& S = st[c.chain];
+        if (S.done) continue;
         const LzChain C = ch[c.chain];
         const int nk = S.j + 1;
         __syncthreads();
-        if (PASS > 0 && threadIdx.x < nk) hs[threadIdx.x] = (PASS == 1) ? S.h1[threadIdx.x] : S.h2[threadIdx.x];
-        __syncthreads();
-        const int end = c.off + c.len;
+        if (PASS > 0 && tid < nk) hs[tid] = (PASS == 1) ? S.h1[tid] : S.h2[tid];
+        const cplx* V = C.V + c.off + tid;
+        cplx* w = C.w + c.off + tid;
         cplx wv[kEpt];
 #pragma unroll
-        for (int e = 0; e < kEpt; ++e) {
-            const int i = c.off + threadIdx.x + e * kLzT;
-            wv[e] = (i < end) ? C.w[i] : cmake(0, 0);
-        }
+        for (int e = 0; e < kEpt; ++e) wv[e] = (tid + e * kLzT < c.len) ? w[e * kLzT] : cmake(0, 0);
+        cplx v[4][kEpt];
+        auto load = [&](int k0) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int e = 0; e < kEpt; ++e)
+                    v[q][e] = (k0 + q < nk && tid + e * kLzT < c.len) ? V[(long long)(k0 + q) * C.n + e * kLzT]
+                                                                      : cmake(0, 0);
+        };
+        __syncthreads();
         if (PASS > 0) {
-            double nr[1] = {0}, ni[1] = {0};
-            for (int k = 0; k < nk; ++k) {
-                const cplx h = hs[k];
-                const cplx* Vk = C.V + (long long)k * C.n;
+            for (int k0 = 0; k0 < nk; k0 += 4) {
+                load(k0);
 #pragma unroll
-                for (int e = 0; e < kEpt; ++e) {
-                    const int i = c.off + threadIdx.x + e * kLzT;
-                    if (i < end) {
-                        const cplx v = Vk[i];
-                        wv[e].x -= v.x * h.x - v.y * h.y;
-                        wv[e].y -= v.x * h.y + v.y * h.x;
-                    }
-                }
-            }
+                for (int q = 0; q < 4; ++q) {
+                    if (k0 + q < nk) {
+                        const cplx h = hs[k0 + q];
 #pragma unroll
-            for (int e = 0; e < kEpt; ++e) {
-                const int i = c.off + threadIdx.x + e * kLzT;
-                if (i < end) {
-                    C.w[i] = wv[e];
-                    nr[0] = fma(wv[e].x, wv[e].x, fma(wv[e].y, wv[e].y, nr[0]));
-                }
-            }
-            if (PASS == 2) block_sum_c<1>(nr, ni, 1, red, part + (long long)t * kPartStride);
-        }
-        if constexpr (PASS < 2) for (int k0 = 0; k0 < nk; k0 += 4) {
-            const int kc = min(4, nk - k0);
-            double ar[4] = {0, 0, 0, 0}, ai[4] = {0, 0, 0, 0};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (q < kc) {
-                    const cplx* Vk = C.V + (long long)(k0 + q) * C.n;
-#pragma unroll
-                    for (int e = 0; e < kEpt; ++e) {
-                        const int i = c.off + threadIdx.x + e * kLzT;
-                        if (i < end) {
-                            const cplx v = Vk[i];   // conj(v) * w
-                            ar[q] = fma(v.x, wv[e].x, fma(v.y, wv[e].y, ar[q]));
-                            ai[q] = fma(v.x, wv[e].y, fma(-v.y, wv[e].x, ai[q]));
+                        for (int e = 0; e < kEpt; ++e) {
+                            wv[e].x -= v[q][e].x * h.x - v[q][e].y * h.y;
+                            wv[e].y -= v[q][e].x * h.y + v[q][e].y * h.x;
                         }
                     }
                 }
             }
-            block_sum_c<4>(ar, ai, kc, red, part + (long long)t * kPartStride + k0);
+            double nr = 0;
+#pragma unroll
+            for (int e = 0; e < kEpt; ++e) {
+                if (tid + e * kLzT < c.len) {
+                    w[e * kLzT] = wv[e];
+                    nr = fma(wv[e].x, wv[e].x, fma(wv[e].y, wv[e].y, nr));
+                }
+            }
+            if (PASS == 2) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) nr += __shfl_xor_sync(0xffffffffu, nr, o);
+                if (lane == 0) red[wid][0] = nr, red[wid][1] = 0;
+            }
+        }
+        if constexpr (PASS < 2) {
+            for (int k0 = 0; k0 < nk; k0 += 4) {
+                load(k0);
+                double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int e = 0; e < kEpt; ++e) {   // conj(v) * w
+                        a[2 * q] = fma(v[q][e].x, wv[e].x, fma(v[q][e].y, wv[e].y, a[2 * q]));
+                        a[2 * q + 1] = fma(v[q][e].x, wv[e].y, fma(-v[q][e].y, wv[e].x, a[2 * q + 1]));
+                    }
+                const double x = warp_sum8(a, lane);
+                if ((lane & 3) == 0) red[wid][2 * k0 + (lane >> 2)] = x;
+            }
+        }
+        __syncthreads();
+        const int ns = PASS < 2 ? 2 * nk : 2;   // doubles summed over the chain
+        double x = 0;
+        double* out = reinterpret_cast<double*>(part + (long long)t * kPartStride);
+        if (tid < ns) {
+#pragma unroll
+            for (int u = 0; u < kLzW; ++u) x += red[u][tid];
+            if (C.ccount > 1) out[tid] = x;
+        }
+        if (!last_of_chain(C.ccount, counters + c.chain)) continue;
+        if (tid < ns) {
+            double y = 0;
+            if (C.ccount > 1) {
+                const double* in = reinterpret_cast<const double*>(part + (long long)C.cstart * kPartStride) + tid;
+#pragma unroll 8
+                for (int q = 0; q < C.ccount; ++q) y += __ldcg(in + (long long)q * 2 * kPartStride);
+            } else {
+                y += x;
+            }
+            if (PASS == 0) reinterpret_cast<double*>(S.h1)[tid] = y;
+            else if (PASS == 1) reinterpret_cast<double*>(S.h2)[tid] = y;
+            else if (tid == 0) {
+                S.wn2 = y;
+                S.mv = 1;
+                S.jv = S.j + 1;
+            }
         }
     }
-}
-
-template <int PASS>
-__global__ void __launch_bounds__(kLzT) lz_cgs_kernel(const VChunk* __restrict__ chunks, const int* __restrict__ nchunks,
-                                                      const LzChain* __restrict__ ch, LzState* __restrict__ st,
-                                                      cplx* __restrict__ part) {
-    cgs_phase<PASS>(chunks, nchunks, ch, st, part, blockIdx.x, gridDim.x);
-}
-
-// Per chain (one warp): h = sum of the chain's chunk partials in chunk order.
-template <int PASS>
-__device__ __forceinline__ void reduce_chain(int c, int lane, const LzChain* __restrict__ ch, LzState* __restrict__ st,
-                                             const cplx* __restrict__ part) {
-    LzState& S = st[c];
-    if (S.done || S.stall) return;
-    const int nk = (PASS < 2) ? S.j + 1 : 1;
-    if (lane >= nk) return;
-    const LzChain C = ch[c];
-    double x = 0, y = 0;
-    for (int q = 0; q < C.ccount; ++q) {
-        const cplx v = part[(long long)(C.cstart + q) * kPartStride + lane];
-        x += v.x;
-        y += v.y;
-    }
-    if (PASS == 0) S.h1[lane] = cmake(x, y);
-    else if (PASS == 1) S.h2[lane] = cmake(x, y);
-    else S.wn2 = x;
-}
-
-template <int PASS>
-__global__ void lz_reduce_kernel(int nchains, const LzChain* __restrict__ ch, LzState* __restrict__ st,
-                                 const cplx* __restrict__ part) {
-    const int c = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
-    if (c < nchains) reduce_chain<PASS>(c, lane, ch, st, part);
 }
 
 // One block per chain: column j of the projected matrix from the
@@ -566,35 +613,21 @@ __global__ void __launch_bounds__(RITZ_THREADS) lz_ritz_kernel(int nchains, cons
     if (c < nchains) ritz_chain(c, w, ch, st, rz);
 }
 
-// V_{j+1} = w / beta_j for the chains that advance.
-__device__ __forceinline__ void next_phase(const VChunk* __restrict__ chunks, const int* __restrict__ nchunks,
-                                                       const LzChain* __restrict__ ch, const LzState* __restrict__ st, int vb, int nvb) {
-    const int total = *nchunks;
-    for (int t = vb; t < total; t += nvb) {
-        const VChunk c = chunks[t];
-        const LzState& S = st[c.chain];
-        if (!S.adv) continue;
-        const LzChain C = ch[c.chain];
-        const double f = 1.0 / S.beta;
-        cplx* vn = C.V + (long long)(S.j + 1) * C.n;
-        for (int i = c.off + threadIdx.x; i < c.off + c.len; i += kLzT) vn[i] = cscale(C.w[i], f);
-    }
-}
-
+// V_{j+1} = w / beta_j.  Whether the chain converged is not known yet: the
+// vector is the next one to expand also after a thick restart, and a chain that
+// turns out to be done leaves it unused.
 __global__ void __launch_bounds__(kLzT) lz_next_kernel(const VChunk* __restrict__ chunks, const int* __restrict__ nchunks,
                                                        const LzChain* __restrict__ ch, const LzState* __restrict__ st) {
-    next_phase(chunks, nchunks, ch, st, blockIdx.x, gridDim.x);
-}
-
-__global__ void lz_inc_kernel(int nchains, LzState* __restrict__ st, int* __restrict__ active) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nchains) return;
-    LzState& S = st[c];
-    if (S.adv) {
-        S.j++;
-        S.adv = 0;
+    const int total = *nchunks;
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+        const VChunk c = chunks[t];
+        const LzState& S = st[c.chain];
+        if (!S.mv) continue;
+        const LzChain C = ch[c.chain];
+        const double f = 1.0 / sqrt(fmax(S.wn2, 0.0));
+        cplx* vn = C.V + (long long)S.jv * C.n;
+        for (int i = c.off + threadIdx.x; i < c.off + c.len; i += kLzT) vn[i] = cscale(C.w[i], f);
     }
-    if (!S.done && !S.stall) atomicAdd(active, 1);
 }
 
 // ---- solve set-up, restarts and the result ------------------------------------
@@ -605,6 +638,7 @@ __global__ void lz_init_kernel(int nchains, const int* __restrict__ solving, LzS
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nchains) return;
     LzState& S = st[c];
+    S.mv = 0;
     if (solving[c] == 2) return;
     const bool start = solving[c] == 1;
     S.j = 0;
@@ -695,6 +729,9 @@ __global__ void lz_norm_kernel(int nchains, const LzChain* __restrict__ ch, LzSt
         if (!(nrm > 1e-280)) {
             S.done = 1;
             S.fail = 1;
+        } else {
+            S.mv = 1;
+            S.jv = 0;
         }
     } else {
         const double e0 = S.energy, ev = S.theta;
@@ -727,96 +764,79 @@ __global__ void __launch_bounds__(kLzT) lz_scale_kernel(const VChunk* __restrict
     }
 }
 
-// ---- thick restart (Wu & Simon 2000), for the chains whose basis is full ---
-// Y_i = V S(:,i) for the `keep` wanted Ritz vectors, Y_keep = w / beta (the
-// residual direction, orthogonal to them).
-__device__ __forceinline__ void restart_form_phase(const VChunk* __restrict__ chunks,
-                                                               const int* __restrict__ nchunks,
-                                                               const LzChain* __restrict__ ch,
-                                                               const LzState* __restrict__ st,
-                                                               const LzRitz* __restrict__ rz, int vb, int nvb) {
+// ---- the end of an iteration, with the thick restart (Wu & Simon 2000) --------
+// A chain that goes on moves to its next vector.  A chain whose basis is full
+// restarts: V_i = V S(:,i) for the `keep` wanted Ritz vectors and V_keep = V_m,
+// the residual direction, orthogonal to them; the projected matrix becomes
+// diag(theta_0 .. theta_{keep-1}) and the expansion continues from V_keep, whose
+// product with the operator is already in w.  After maxit restarts the solve
+// fails (info -14 of the reference, core.f95:2565-2607).  An element of the new
+// basis needs that element of the old one only, so the basis is rewritten in
+// place; the chain's last chunk changes its state.
+__global__ void __launch_bounds__(kLzT) lz_advance_kernel(const VChunk* __restrict__ chunks,
+                                                          const int* __restrict__ nchunks,
+                                                          const LzChain* __restrict__ ch, LzState* __restrict__ st,
+                                                          LzRitz* __restrict__ rz, int* __restrict__ counters,
+                                                          int* __restrict__ active) {
     __shared__ double ss[kKeepMax * kMaxKrylov];
     const int total = *nchunks;
-    for (int t = vb; t < total; t += nvb) {
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
         const VChunk c = chunks[t];
-        const LzState& S = st[c.chain];
-        if (S.done || !S.stall) continue;
+        LzState& S = st[c.chain];
         const LzChain C = ch[c.chain];
+        if (S.done || !S.stall) {
+            if (t == C.cstart && threadIdx.x == 0) {
+                S.mv = 0;
+                if (S.adv) {
+                    S.j++;
+                    S.adv = 0;
+                }
+                if (!S.done) atomicAdd(active, 1);
+            }
+            continue;
+        }
         const int m = S.j + 1;
         __syncthreads();
         for (int e = threadIdx.x; e < C.keep * kMaxKrylov; e += kLzT) ss[e] = rz[c.chain].S[e];
         __syncthreads();
-        const double fb = 1.0 / S.beta;
         for (int i = c.off + threadIdx.x; i < c.off + c.len; i += kLzT) {
-            for (int q = 0; q < C.keep; ++q) {
-                double vr = 0, vi = 0;
-                for (int k = 0; k < m; ++k) {
-                    const cplx b = C.V[(long long)k * C.n + i];
-                    const double f = ss[q * kMaxKrylov + k];
-                    vr = fma(f, b.x, vr);
-                    vi = fma(f, b.y, vi);
+            double vr[kKeepMax], vi[kKeepMax];
+#pragma unroll
+            for (int q = 0; q < kKeepMax; ++q) vr[q] = vi[q] = 0;
+#pragma unroll 4
+            for (int k = 0; k < m; ++k) {
+                const cplx b = C.V[(long long)k * C.n + i];
+#pragma unroll
+                for (int q = 0; q < kKeepMax; ++q) {
+                    if (q < C.keep) {
+                        const double f = ss[q * kMaxKrylov + k];
+                        vr[q] = fma(f, b.x, vr[q]);
+                        vi[q] = fma(f, b.y, vi[q]);
+                    }
                 }
-                C.Y[(long long)q * C.n + i] = cmake(vr, vi);
             }
-            C.Y[(long long)C.keep * C.n + i] = cscale(C.w[i], fb);
+            const cplx last = C.V[(long long)m * C.n + i];
+#pragma unroll
+            for (int q = 0; q < kKeepMax; ++q)
+                if (q < C.keep) C.V[(long long)q * C.n + i] = cmake(vr[q], vi[q]);
+            C.V[(long long)C.keep * C.n + i] = last;
         }
-    }
-}
-
-__global__ void __launch_bounds__(kLzT) lz_restart_form_kernel(const VChunk* __restrict__ chunks,
-                                                               const int* __restrict__ nchunks,
-                                                               const LzChain* __restrict__ ch,
-                                                               const LzState* __restrict__ st,
-                                                               const LzRitz* __restrict__ rz) {
-    restart_form_phase(chunks, nchunks, ch, st, rz, blockIdx.x, gridDim.x);
-}
-
-// V_0..V_keep = Y_0..Y_keep.
-__device__ __forceinline__ void restart_copy_phase(const VChunk* __restrict__ chunks,
-                                                               const int* __restrict__ nchunks,
-                                                               const LzChain* __restrict__ ch,
-                                                               const LzState* __restrict__ st, int vb, int nvb) {
-    const int total = *nchunks;
-    for (int t = vb; t < total; t += nvb) {
-        const VChunk c = chunks[t];
-        const LzState& S = st[c.chain];
-        if (S.done || !S.stall) continue;
-        const LzChain C = ch[c.chain];
-        for (int q = 0; q <= C.keep; ++q)
-            for (int i = c.off + threadIdx.x; i < c.off + c.len; i += kLzT)
-                C.V[(long long)q * C.n + i] = C.Y[(long long)q * C.n + i];
-    }
-}
-
-__global__ void __launch_bounds__(kLzT) lz_restart_copy_kernel(const VChunk* __restrict__ chunks,
-                                                               const int* __restrict__ nchunks,
-                                                               const LzChain* __restrict__ ch,
-                                                               const LzState* __restrict__ st) {
-    restart_copy_phase(chunks, nchunks, ch, st, blockIdx.x, gridDim.x);
-}
-
-// Per chain (one block): the projected matrix becomes diag(theta_0 ..
-// theta_{keep-1}) and the expansion continues from V_keep; after maxit
-// restarts the solve fails (info -14 of the reference, core.f95:2565-2607).
-__global__ void lz_restart_state_kernel(int nchains, const LzChain* __restrict__ ch, LzState* __restrict__ st,
-                                        LzRitz* __restrict__ rz) {
-    const int c = blockIdx.x;
-    if (c >= nchains) return;
-    LzState& S = st[c];
-    if (S.done || !S.stall) return;
-    const LzChain C = ch[c];
-    const bool fail = S.restarts + 1 >= C.maxit;
-    if (!fail) ritz_restart_state<kMaxKrylov>(C.keep, rz[c].theta, rz[c].state);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (fail) {
-            S.done = 1;
-            S.fail = 1;
-        } else {
-            S.restarts++;
-            S.j = C.keep;
+        if (!last_of_chain(C.ccount, counters + c.chain)) continue;
+        const bool fail = S.restarts + 1 >= C.maxit;
+        if (!fail) ritz_restart_state<kMaxKrylov>(C.keep, rz[c.chain].theta, rz[c.chain].state);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            S.mv = 0;
+            S.stall = 0;
+            if (fail) {
+                S.done = 1;
+                S.fail = 1;
+            } else {
+                S.restarts++;
+                S.j = C.keep;
+                atomicAdd(active, 1);
+            }
         }
-        S.stall = 0;
     }
 }
 
@@ -1258,7 +1278,7 @@ struct ChainHost {
     std::vector<int> phys, bonds;
     std::vector<MpoDev> ops;
     std::vector<cplx*> site, L, R;
-    cplx *spare = nullptr, *T = nullptr, *U = nullptr, *V = nullptr, *w = nullptr, *Y = nullptr;
+    cplx *spare = nullptr, *T = nullptr, *U = nullptr, *V = nullptr, *w = nullptr;
     cplx *X = nullptr, *Q = nullptr, *tau = nullptr, *rbuf = nullptr;
     size_t max_site = 0;
     // sweep state
@@ -1293,7 +1313,7 @@ struct Engine {
     DevArray<LzChain> d_lz;
     DevArray<LzState> d_st;
     DevArray<LzRitz> d_rz;
-    DevArray<int> d_solving, d_active, d_finished;
+    DevArray<int> d_solving, d_active, d_finished, d_arrived;
     DevArray<double> d_energy;
     DevArray<cplx> d_part, d_part_n;
     DevArray<NormJob> d_norm_jobs;
@@ -1320,10 +1340,15 @@ struct Engine {
     double seconds = 0, seconds_moves = 0, seconds_solves = 0;   // the last two with time_phases
     double seconds_replays = 0;   // device time of the Lanczos graph replays (time_phases)
     cudaEvent_t ev_a = nullptr, ev_b = nullptr;
+    cudaStream_t side = nullptr;   // capture only: the projected problems' branch
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 
     ~Engine() {
         if (ev_a) cudaEventDestroy(ev_a);
         if (ev_b) cudaEventDestroy(ev_b);
+        if (ev_fork) cudaEventDestroy(ev_fork);
+        if (ev_join) cudaEventDestroy(ev_join);
+        if (side) cudaStreamDestroy(side);
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
         if (graph) cudaGraphDestroy(graph);
         if (pool) cudaFree(pool);
@@ -1398,7 +1423,6 @@ struct Engine {
                      + env                                                // environments
                      + align_up(mt) + align_up(mu)                        // T, U
                      + (size_t)(kMaxKrylov + 2) * align_up(ms)            // V, w
-                     + (size_t)(kKeepMax + 1) * align_up(ms)              // Y (thick restart)
                      + 2 * align_up(ms) + align_up(mb) + align_up(mb * mb);   // X, Q, tau, R
         }
         pool_bytes = total * sizeof(cplx) + mpo_bytes + 4096;
@@ -1446,7 +1470,6 @@ struct Engine {
             ch.U = take(mu);
             ch.V = take((size_t)(kMaxKrylov + 1) * align_up(ch.max_site));
             ch.w = take(ch.max_site);
-            ch.Y = take((size_t)(kKeepMax + 1) * align_up(ch.max_site));
             ch.X = take(ch.max_site);
             ch.Q = take(ch.max_site);
             ch.tau = take(mb);
@@ -1488,6 +1511,7 @@ struct Engine {
         d_finished.reserve(B);
         d_energy.reserve(B);
         d_active.reserve(1);
+        d_arrived.reserve(B);
         d_part.reserve(nchunk_cap * kPartStride);
         d_part_n.reserve(nchunk_cap * kPartStride);
         d_norm_jobs.reserve(B);
@@ -1502,13 +1526,14 @@ struct Engine {
         NC_CUDA(cudaMallocHost(&h_energy, B * sizeof(double)));
         NC_CUDA(cudaMallocHost(&h_state, B * sizeof(LzState)));
         NC_CUDA(cudaMemsetAsync(d_st.p, 0, B * sizeof(LzState), stream));
+        NC_CUDA(cudaMemsetAsync(d_arrived.p, 0, B * sizeof(int), stream));
         // persistent grids from the occupancy of each kernel
         int occ = 0;
         NC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, grouped_gemm_kernel, kGemmThreads, kGemmSmem));
         grid_gemm = sms * std::max(1, occ);
         NC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, grouped_mix_kernel, 256, 0));
         grid_mix = sms * std::max(1, occ);
-        NC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, lz_cgs_kernel<1>, kLzT, 0));
+        NC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, lz_next_kernel, kLzT, 0));
         grid_vec = sms * std::max(1, occ);
         NC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batched_qr_kernel, kQrThreads, 0));
         grid_qr = sms * std::max(1, occ);
@@ -1759,36 +1784,53 @@ struct Engine {
         run_normalise();
     }
 
-    void capture_graph() {
-        if (graph_exec) return;
-        const int B = (int)chains.size();
-        const int cb = (B + 7) / 8, tb = (B + 255) / 256;
+    // w = H_eff V_jv of every chain with mv set.
+    void launch_matvec() {
         LzState* st = d_st.p;
-        NC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         grouped_gemm_kernel<<<grid_gemm, kGemmThreads, kGemmSmem, stream>>>(g_a.d_probs.p, g_a.d_prefix.p,
                                                                              g_a.d_tile.p, g_a.d_count.p, st);
         grouped_mix_kernel<<<grid_mix, 256, 0, stream>>>(m_h.d_probs.p, m_h.d_items.p, m_h.d_count.p, st);
         grouped_gemm_kernel<<<grid_gemm, kGemmThreads, kGemmSmem, stream>>>(g_c.d_probs.p, g_c.d_prefix.p,
                                                                              g_c.d_tile.p, g_c.d_count.p, st);
-        lz_cgs_kernel<0><<<grid_vec, kLzT, 0, stream>>>(lz_chunks.d.p, lz_chunks.d_count.p, d_lz.p, st, d_part.p);
-        lz_reduce_kernel<0><<<cb, 256, 0, stream>>>(B, d_lz.p, st, d_part.p);
-        lz_cgs_kernel<1><<<grid_vec, kLzT, 0, stream>>>(lz_chunks.d.p, lz_chunks.d_count.p, d_lz.p, st, d_part.p);
-        lz_reduce_kernel<1><<<cb, 256, 0, stream>>>(B, d_lz.p, st, d_part.p);
-        lz_cgs_kernel<2><<<grid_vec, kLzT, 0, stream>>>(lz_chunks.d.p, lz_chunks.d_count.p, d_lz.p, st, d_part.p);
-        lz_reduce_kernel<2><<<cb, 256, 0, stream>>>(B, d_lz.p, st, d_part.p);
-        lz_ritz_kernel<<<B, RITZ_THREADS, 0, stream>>>(B, d_lz.p, st, d_rz.p, d_active.p);
-        lz_next_kernel<<<grid_vec, kLzT, 0, stream>>>(lz_chunks.d.p, lz_chunks.d_count.p, d_lz.p, st);
-        // thick restart of the chains whose basis filled in this iteration
-        lz_restart_form_kernel<<<grid_vec, kLzT, 0, stream>>>(lz_chunks.d.p, lz_chunks.d_count.p, d_lz.p, st, d_rz.p);
-        lz_restart_copy_kernel<<<grid_vec, kLzT, 0, stream>>>(lz_chunks.d.p, lz_chunks.d_count.p, d_lz.p, st);
-        lz_restart_state_kernel<<<B, 32, 0, stream>>>(B, d_lz.p, st, d_rz.p);
-        lz_inc_kernel<<<tb, 256, 0, stream>>>(B, st, d_active.p);
+    }
+
+    // One Lanczos iteration.  It begins with w = H_eff V_j in place and ends
+    // with the next vector's product: the next vector is w / |w| whatever the
+    // projected problem says (also after a thick restart, where it becomes
+    // V_keep), so the projected problem, a chain of dependent FP64 operations
+    // on one block per chain, runs beside that product.  The price is one
+    // unused product at the end of a solve.  B200, against fifteen kernels in a
+    // row: 12 chains of 8 to 10 sites, chi <= 16, three sweeps 220 -> 185 ms;
+    // 256 chains of 8 to 48 sites, chi <= 128, 3.8 -> 4.6 chains a second.
+    void capture_graph() {
+        if (graph_exec) return;
+        const int B = (int)chains.size();
+        LzState* st = d_st.p;
+        const VChunk* vc = lz_chunks.d.p;
+        const int* nvc = lz_chunks.d_count.p;
+        if (!side) {
+            NC_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+            NC_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+            NC_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+        }
+        NC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+        lz_cgs_kernel<0><<<grid_vec, kLzT, 0, stream>>>(vc, nvc, d_lz.p, st, d_part.p, d_arrived.p);
+        lz_cgs_kernel<1><<<grid_vec, kLzT, 0, stream>>>(vc, nvc, d_lz.p, st, d_part.p, d_arrived.p);
+        lz_cgs_kernel<2><<<grid_vec, kLzT, 0, stream>>>(vc, nvc, d_lz.p, st, d_part.p, d_arrived.p);
+        NC_CUDA(cudaEventRecord(ev_fork, stream));
+        NC_CUDA(cudaStreamWaitEvent(side, ev_fork, 0));
+        lz_ritz_kernel<<<B, RITZ_THREADS, 0, side>>>(B, d_lz.p, st, d_rz.p, d_active.p);
+        NC_CUDA(cudaEventRecord(ev_join, side));
+        lz_next_kernel<<<grid_vec, kLzT, 0, stream>>>(vc, nvc, d_lz.p, st);
+        launch_matvec();
+        NC_CUDA(cudaStreamWaitEvent(stream, ev_join, 0));
+        lz_advance_kernel<<<grid_vec, kLzT, 0, stream>>>(vc, nvc, d_lz.p, st, d_rz.p, d_arrived.p, d_active.p);
         cudaError_t e = cudaStreamEndCapture(stream, &graph);
         NC_CUDA(e);
         NC_CHECK_LAUNCH();
         NC_CUDA(cudaGraphInstantiate(&graph_exec, graph, 0));
     }
-    static constexpr int kGraphKernels = 15;
+    static constexpr int kGraphKernels = 9;
 
     int read_active() {
         NC_CUDA(cudaMemcpyAsync(h_active, d_active.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
@@ -1839,7 +1881,6 @@ struct Engine {
             z.cstart = r.first; z.ccount = r.second;
             z.m_max = (int)opt.krylov_dimension;
             z.keep = std::max(1, std::min(std::max(4, z.m_max / 3), z.m_max - 2));
-            z.Y = ch.Y;
             z.maxit = (int)std::max<uint32_t>(1, opt.maximum_number_of_iterations);
             h_solving[c] = flag;
         };
@@ -1858,8 +1899,12 @@ struct Engine {
                                                          d_part.p);
         lz_norm_kernel<0><<<tb, 256, 0, stream>>>(B, d_lz.p, st, d_solving.p, d_part.p, sanity);
         lz_scale_kernel<0><<<grid_vec, kLzT, 0, stream>>>(lz_chunks.d.p, lz_chunks.d_count.p, d_lz.p, st, d_solving.p);
-        NC_CHECK_LAUNCH();
         launches += 4;
+        if (!starting.empty()) {   // a continuing chain's product is in place
+            launch_matvec();
+            launches += 3;
+        }
+        NC_CHECK_LAUNCH();
         const int check_every = 4;
         uint64_t iters = 0;
         if (opt.time_phases) {
