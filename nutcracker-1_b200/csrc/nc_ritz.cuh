@@ -17,19 +17,22 @@
 // every rotation.
 //
 // What bounds it is latency: a sweep is m - 1 rounds, each the chain
-// (rotation angles) -> (rotated blocks), and a site solve waits for it at
+// (rotation angles) -> (rotated blocks of A), and a solve waits for it at
 // every Lanczos step.  So the block splits each round over its threads: one
-// warp computes the angles of the round's disjoint pairs, then every 2 x 2
-// block (pair r, pair q) of A and every (row, pair) of Z belongs to one
-// thread, in place, with one barrier after each half; whether a sweep is
-// needed at all is asked of all pairs at once instead of by a last sweep that
-// rotates nothing.  Every element goes through the same operations in the
-// same order as in a one-warp update, so the Ritz pairs are the same bits for
-// any number of threads.  Measured on a B200 (site solve of a 48 x 48 x 2
-// site, 24-vector basis, mean over the solve): one warp 148 us an update, this
-// form 65 us; the solve 9.5 -> 6.8 ms.  Starting the angles from FP32 values
-// with FP64 Newton steps instead of the divisions and square roots gains
-// another 3% of a solve and changes the rounding, so it is not done.
+// warp computes the angles of the round's disjoint pairs while the others
+// apply the round before to Z, which no angle depends on; then every 2 x 2
+// block (pair r, pair q) of A belongs to one thread, in place.  Which block,
+// rows and pairs a thread has is the same in every round and computed once.
+// Whether a sweep is needed at all is asked of all pairs at once instead of by
+// a last sweep that rotates nothing.  Every element goes through the same
+// operations in the same order as in a one-warp update, so the Ritz pairs are
+// the same bits for any number of threads.  Measured on a B200: one warp
+// 148 us an update (mean over the solve of a 48 x 48 x 2 site, 24-vector
+// basis), 65 us with A and Z rotated together between the angles, that is
+// 2280 clocks a round at m = 24 and 1950 at m = 20, now 1550 and 1510; most of
+// that is the angles' three divisions and two square roots in a row.
+// Starting them from FP32 values with FP64 Newton steps gains another 3% of a
+// solve and changes the rounding, so it is not done.
 #pragma once
 
 #include "nc_common.cuh"
@@ -50,9 +53,9 @@ template <int MAXT>
 struct RitzSmem {
     double A[MAXT][MAXT + 1], Z[MAXT][MAXT + 1];
     double tcol[MAXT];
-    double cs[MAXT / 2], sn[MAXT / 2];
+    double cs[2][MAXT / 2], sn[2][MAXT / 2];   // angles of a round and of the one before
     int perm[MAXT];
-    int rotated;
+    int rotated[2];
 };
 
 // Whether the pair (app, aqq) still needs its rotation: apq above the
@@ -122,74 +125,91 @@ __device__ RitzResult ritz_update_block(RitzSmem<MAXT>& w, int m, double* __rest
     }
     if (tid == 0) w.A[m - 1][m - 1] = w.tcol[m - 1];
     __syncthreads();
-    const int nA = np * np, nZ = np * m;
+    // Thread-constant work: elements of the check, one block of A, (row, pair) of Z.
+    static_assert(MAXT * MAXT / 4 <= RITZ_THREADS, "one block of A per thread");
+    constexpr int NCHK = (MAXT * MAXT / 2 + RITZ_THREADS - 1) / RITZ_THREADS;
+    constexpr int ZT = RITZ_THREADS - 32, NROT = (MAXT * MAXT / 2 + ZT - 1) / ZT;
+    int ca[NCHK], cb[NCHK], zi[NROT], zq[NROT];
+#pragma unroll
+    for (int u = 0; u < NCHK; ++u) {
+        const int e = tid + u * RITZ_THREADS, s = e / np, r = e - s * np;
+        ca[u] = r == 0 ? mp - 1 : (s + r) % (mp - 1);
+        cb[u] = s >= mp - 1 ? -1 : r == 0 ? s : (s - r + mp - 1) % (mp - 1);
+    }
+#pragma unroll
+    for (int u = 0; u < NROT; ++u) {
+        const int f = tid - 32 + u * ZT;
+        zi[u] = f >= 0 ? f / np : m;
+        zq[u] = f - zi[u] * np;
+    }
+    const int rA = tid / np, qA = tid - rA * np;
+    // round s's pairs: r = 0 (mp-1, s), r > 0 (s + r, s - r) mod mp-1
+    auto first = [&](int s, int r) { const int a = s + r; return r == 0 ? mp - 1 : (a >= mp - 1 ? a - (mp - 1) : a); };
+    auto second = [&](int s, int r) { const int b = s - r; return r == 0 ? s : (b < 0 ? b + (mp - 1) : b); };
+    // columns of pair q in row i of Z, round s
+    auto rotate_z = [&](int s) {
+        if (!w.rotated[s & 1]) return;
+#pragma unroll
+        for (int u = 0; u < NROT; ++u) {
+            if (zi[u] >= m) continue;
+            const int i = zi[u], a = first(s, zq[u]), b = second(s, zq[u]);
+            const double cq = w.cs[s & 1][zq[u]], sq = w.sn[s & 1][zq[u]], va = w.Z[i][a], vb = w.Z[i][b];
+            if (sq == 0.0) continue;
+            w.Z[i][a] = cq * va - sq * vb;
+            w.Z[i][b] = sq * va + cq * vb;
+        }
+    };
     int sweep = 0;
     for (; sweep < 30; ++sweep) {
-        bool any = false;   // a sweep is needed while any pair would rotate
-        for (int e = tid; e < (mp - 1) * np; e += RITZ_THREADS) {   // asked of the same element as in its round
-            const int s = e / np, r = e - s * np;
-            const int a = r == 0 ? mp - 1 : (s + r) % (mp - 1), b = r == 0 ? s : (s - r + mp - 1) % (mp - 1);
-            any |= ritz_rotates(w.A[a][b], w.A[a][a], w.A[b][b]);
-        }
+        bool any = false;   // a sweep is needed while any pair would rotate; asked of the same element as in its round
+#pragma unroll
+        for (int u = 0; u < NCHK; ++u)
+            if (cb[u] >= 0) any |= ritz_rotates(w.A[ca[u]][cb[u]], w.A[ca[u]][ca[u]], w.A[cb[u]][cb[u]]);
         if (!__syncthreads_or(any)) break;
         for (int s = 0; s < mp - 1; ++s) {
-            // the round's pairs: r = 0 (mp-1, s), r > 0 (s + r, s - r) mod mp-1
-            auto first = [&](int r) { const int a = s + r; return r == 0 ? mp - 1 : (a >= mp - 1 ? a - (mp - 1) : a); };
-            auto second = [&](int r) { const int b = s - r; return r == 0 ? s : (b < 0 ? b + (mp - 1) : b); };
             if (tid < 32) {
                 double c = 1.0, sv = 0.0;
                 bool rot = false;
                 if (tid < np) {
-                    const int a = first(tid), b = second(tid);
+                    const int a = first(s, tid), b = second(s, tid);
                     const double apq = w.A[a][b], app = w.A[a][a], aqq = w.A[b][b];
                     rot = ritz_rotates(apq, app, aqq);
                     if (rot) ritz_rotation(apq, app, aqq, c, sv);
-                    w.cs[tid] = c;
-                    w.sn[tid] = sv;
+                    w.cs[s & 1][tid] = c;
+                    w.sn[s & 1][tid] = sv;
                 }
                 rot = __any_sync(0xffffffffu, rot);
-                if (tid == 0) w.rotated = rot;
+                if (tid == 0) w.rotated[s & 1] = rot;
+            } else if (s > 0) {
+                rotate_z(s - 1);
             }
             __syncthreads();
-            if (!w.rotated) {
-                __syncthreads();   // the flag is rewritten by the next round
-                continue;
-            }
-            for (int e = tid; e < nA + nZ; e += RITZ_THREADS) {
-                if (e < nA) {   // block (rows of pair r, columns of pair q)
-                    const int r = e / np, q = e - r * np;
-                    const double cr = w.cs[r], sr = w.sn[r], cq = w.cs[q], sq = w.sn[q];
-                    const int ar = first(r), br = second(r), aq = first(q), bq = second(q);
-                    double x00 = w.A[ar][aq], x01 = w.A[ar][bq], x10 = w.A[br][aq], x11 = w.A[br][bq];
-                    if (sr != 0.0) {   // rows
-                        const double y0 = x00, y1 = x01;
-                        x00 = cr * y0 - sr * x10;
-                        x01 = cr * y1 - sr * x11;
-                        x10 = sr * y0 + cr * x10;
-                        x11 = sr * y1 + cr * x11;
-                    }
-                    if (sq != 0.0) {   // columns
-                        const double y0 = x00, y1 = x10;
-                        x00 = cq * y0 - sq * x01;
-                        x10 = cq * y1 - sq * x11;
-                        x01 = sq * y0 + cq * x01;
-                        x11 = sq * y1 + cq * x11;
-                    }
-                    w.A[ar][aq] = x00; w.A[ar][bq] = x01; w.A[br][aq] = x10; w.A[br][bq] = x11;
-                } else {        // columns of pair q in row i of Z
-                    const int f = e - nA, i = f / np, q = f - i * np;
-                    const double sq = w.sn[q];
-                    if (sq == 0.0) continue;
-                    const double cq = w.cs[q];
-                    const int a = first(q), b = second(q);
-                    const double va = w.Z[i][a], vb = w.Z[i][b];
-                    w.Z[i][a] = cq * va - sq * vb;
-                    w.Z[i][b] = sq * va + cq * vb;
+            if (!w.rotated[s & 1]) continue;
+            if (rA < np) {   // block (rows of pair rA, columns of pair qA)
+                const double cr = w.cs[s & 1][rA], sr = w.sn[s & 1][rA], cq = w.cs[s & 1][qA], sq = w.sn[s & 1][qA];
+                const int ar = first(s, rA), br = second(s, rA), aq = first(s, qA), bq = second(s, qA);
+                double x00 = w.A[ar][aq], x01 = w.A[ar][bq], x10 = w.A[br][aq], x11 = w.A[br][bq];
+                if (sr != 0.0) {   // rows
+                    const double y0 = x00, y1 = x01;
+                    x00 = cr * y0 - sr * x10;
+                    x01 = cr * y1 - sr * x11;
+                    x10 = sr * y0 + cr * x10;
+                    x11 = sr * y1 + cr * x11;
                 }
+                if (sq != 0.0) {   // columns
+                    const double y0 = x00, y1 = x10;
+                    x00 = cq * y0 - sq * x01;
+                    x10 = cq * y1 - sq * x11;
+                    x01 = sq * y0 + cq * x01;
+                    x11 = sq * y1 + cq * x11;
+                }
+                w.A[ar][aq] = x00; w.A[ar][bq] = x01; w.A[br][aq] = x10; w.A[br][bq] = x11;
             }
             __syncthreads();
         }
+        if (tid >= 32) rotate_z(mp - 2);
     }
+    __syncthreads();
     // order the m genuine Ritz values by rank (a padding direction, if any, is index m)
     if (tid < m) w.perm[tid] = tid;
     __syncthreads();
