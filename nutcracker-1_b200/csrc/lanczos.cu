@@ -278,7 +278,8 @@ constexpr int RITZ_STATE = 2 * MAXT * MAXT;
 
 struct RitzOut {
     double theta, res, beta, tnorm;
-    int sweeps, pad;
+    int sweeps;
+    unsigned ticket;   // in host memory: written after the rest
 };
 
 // after a thick restart: A = diag(theta_0 .. theta_{k-1}), Z = I
@@ -287,23 +288,27 @@ __global__ void restart_t_kernel(int k, const double* __restrict__ theta, double
 }
 
 // Adds column m-1 of T to the kept decomposition and diagonalises (one block);
-// theta[] and S (m x m complex, column-major) receive the ordered Ritz pairs,
-// out the wanted pair's value and Ritz estimate.
+// theta[] and S (m x m complex, column-major) receive the ordered Ritz pairs.
+// The wanted pair's value and Ritz estimate go straight to pinned host memory,
+// marked with `ticket`: a host that watches the mark knows them about a
+// microsecond after the kernel wrote them, against ten for a copy and an event.
 __global__ void __launch_bounds__(RITZ_THREADS)
 ritz_kernel(int m, double* __restrict__ state, const cplx* __restrict__ h1, const cplx* __restrict__ h2,
-            const cplx* __restrict__ nrm2, int which, RitzOut* __restrict__ out, cplx* __restrict__ S,
-            double* __restrict__ theta) {
+            const cplx* __restrict__ nrm2, int which, volatile RitzOut* __restrict__ out, unsigned ticket,
+            cplx* __restrict__ S, double* __restrict__ theta) {
     __shared__ RitzSmem<MAXT> w;
     const RitzResult r = ritz_update_block<MAXT, true>(w, m, state, h1, h2, nrm2[0].x, which, S, m, theta);
+    __syncthreads();   // the mark also stands for the block's other stores
     if (threadIdx.x == 0) {
         out->theta = r.theta;
         out->res = r.res;
         out->beta = r.beta;
         out->tnorm = r.tnorm;
         out->sweeps = r.sweeps;
+        __threadfence_system();
+        out->ticket = ticket;
     }
 }
-
 
 __global__ void scale_by_inv_sqrt(long long n, const cplx* __restrict__ nrm2, const cplx* __restrict__ in,
                                   cplx* __restrict__ out) {
@@ -427,44 +432,64 @@ struct Filter {
     }
 };
 
-// The thread's second stream, on which a projected problem runs beside the
-// next step, with its reading.  Whatever ends the solve, nothing of it is in
-// flight afterwards (its buffers go back to the arena).
+// The projected problem's launch and reading, on the context's stream or on
+// the thread's second one, where it runs beside the next step.  Whatever ends
+// the solve, nothing of it is in flight afterwards (its buffers go back to the
+// arena).
 class RitzLane {
    public:
-    explicit RitzLane(Context& c) : ctx_(c) {}
+    explicit RitzLane(Context& c)
+        : ctx_(c), out_(reinterpret_cast<RitzOut*>(static_cast<char*>(c.pinned) + c.pinned_bytes / 2)) {}
     ~RitzLane() {
-        if (busy_) cudaStreamSynchronize(ctx_.ritz_stream);
+        if (on_) cudaStreamSynchronize(on_);
     }
     RitzLane(const RitzLane&) = delete;
     RitzLane& operator=(const RitzLane&) = delete;
-    // The stream, behind everything enqueued on the context's stream so far.
-    cudaStream_t begin() {
-        if (!ctx_.ritz_stream) {
-            NC_CUDA(cudaEventCreateWithFlags(&ctx_.ritz_ready, cudaEventDisableTiming));
+    // `beside`: on the second stream, behind everything enqueued so far.
+    void launch(bool beside, int m, double* state, const cplx* h1, const cplx* h2, const cplx* nr, int which, cplx* S,
+                double* theta) {
+        if (!ctx_.ritz_done)
             NC_CUDA(cudaEventCreateWithFlags(&ctx_.ritz_done,
                                              cudaEventDisableTiming | (ctx_.blocking_sync ? cudaEventBlockingSync : 0)));
+        if (beside && !ctx_.ritz_stream) {
+            NC_CUDA(cudaEventCreateWithFlags(&ctx_.ritz_ready, cudaEventDisableTiming));
             NC_CUDA(cudaStreamCreateWithFlags(&ctx_.ritz_stream, cudaStreamNonBlocking));
         }
-        NC_CUDA(cudaEventRecord(ctx_.ritz_ready, ctx_.stream));
-        NC_CUDA(cudaStreamWaitEvent(ctx_.ritz_stream, ctx_.ritz_ready, 0));
-        busy_ = true;
-        return ctx_.ritz_stream;
+        if (beside) {
+            NC_CUDA(cudaEventRecord(ctx_.ritz_ready, ctx_.stream));
+            NC_CUDA(cudaStreamWaitEvent(ctx_.ritz_stream, ctx_.ritz_ready, 0));
+        }
+        out_->ticket = ctx_.ritz_ticket++;   // no kernel writes it now: the last one's result was taken
+        on_ = beside ? ctx_.ritz_stream : ctx_.stream;
+        ritz_kernel<<<1, RITZ_THREADS, 0, on_>>>(m, state, h1, h2, nr, which, out_, ctx_.ritz_ticket, S, theta);
+        NC_CHECK_LAUNCH();
+        ctx_.launches++;
+        if (ctx_.blocking_sync) NC_CUDA(cudaEventRecord(ctx_.ritz_done, on_));
     }
-    void read(const void* dev, size_t bytes) {
-        NC_CUDA(cudaMemcpyAsync(slot(), dev, bytes, cudaMemcpyDeviceToHost, ctx_.ritz_stream));
-        NC_CUDA(cudaEventRecord(ctx_.ritz_done, ctx_.ritz_stream));
-    }
-    void wait(void* host, size_t bytes) {
-        NC_CUDA(cudaEventSynchronize(ctx_.ritz_done));
-        busy_ = false;
-        memcpy(host, slot(), bytes);
+    // A thread that may use its core watches the mark, with a look at the
+    // stream now and then (an error ends the wait); one that shares it sleeps.
+    RitzOut wait() {
+        if (ctx_.blocking_sync) {
+            NC_CUDA(cudaEventSynchronize(ctx_.ritz_done));
+        } else {
+            const volatile unsigned* mark = &out_->ticket;
+            for (unsigned spins = 1; *mark != ctx_.ritz_ticket; ++spins) {
+                if (spins % 4096 != 0) continue;
+                const cudaError_t e = cudaStreamQuery(on_);
+                if (e == cudaErrorNotReady) continue;
+                NC_CUDA(e);
+                if (*mark != ctx_.ritz_ticket) throw Error(NC_ERR_CUDA, "projected problem: no result");
+            }
+            std::atomic_thread_fence(std::memory_order_acquire);
+        }
+        on_ = nullptr;
+        return *out_;
     }
 
    private:
-    char* slot() const { return static_cast<char*>(ctx_.pinned) + ctx_.pinned_bytes / 2; }
     Context& ctx_;
-    bool busy_ = false;
+    RitzOut* out_;   // pinned
+    cudaStream_t on_ = nullptr;   // where a launch is in flight
 };
 
 }  // namespace
@@ -537,7 +562,6 @@ int optimize_site(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L
     struct Step {
         cplx *h1, *h2, *nr, *S;
         double* theta;
-        RitzOut* ro;
     } steps[2];
     for (Step& q : steps) {
         q.h1 = ctx.arena.alloc_n<cplx>(m_max + 1);
@@ -545,7 +569,6 @@ int optimize_site(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L
         q.nr = ctx.arena.alloc_n<cplx>(1);
         q.S = ctx.arena.alloc_n<cplx>(MAXT * MAXT);
         q.theta = ctx.arena.alloc_n<double>(MAXT);
-        q.ro = ctx.arena.alloc_n<RitzOut>(1);
     }
     double* T = ctx.arena.alloc_n<double>(RITZ_STATE);   // kept eigen-decomposition of T
 
@@ -610,7 +633,9 @@ int optimize_site(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L
     // stream of its own and the next step starts beside it; a step that turns
     // out not to be needed is dropped (the result only reads V_0 .. V_j).  The
     // residual rule keeps that rare: a step seldom gains a factor of 30.  Site
-    // solve 48 x 48 x 2: 5.6 -> 3.9 ms.
+    // solve 48 x 48 x 2: 5.6 -> 3.9 ms; a 20-site sweep, chi <= 64, whose steps
+    // are as long as the projected problem, 189 -> 146 ms, and 125 -> 115 ms
+    // when the result no longer came by a copy and an event.
     RitzLane lane(ctx);
     constexpr int kAheadFrom = 6;
     constexpr long long kAheadElems = 1LL << 17;
@@ -624,22 +649,12 @@ int optimize_site(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L
         ++st.matvecs;
         const bool ahead = !mixed && n <= kAheadElems && j + 1 >= kAheadFrom && j + 1 < m_max && j + 1 < orth_dim &&
                            last_ratio > 30.0;
-        RitzOut rr;
+        lane.launch(ahead, j + 1, T, q.h1, q.h2, q.nr, which, q.S, q.theta);
         if (ahead) {
-            cudaStream_t rs = lane.begin();
-            ritz_kernel<<<1, RITZ_THREADS, 0, rs>>>(j + 1, T, q.h1, q.h2, q.nr, which, q.ro, q.S, q.theta);
-            NC_CHECK_LAUNCH();
-            ctx.launches++;
-            lane.read(q.ro, sizeof(RitzOut));
             next_vector(j, q);
             expand(j + 1, qn);
-            lane.wait(&rr, sizeof(RitzOut));
-        } else {
-            ritz_kernel<<<1, RITZ_THREADS, 0, ctx.stream>>>(j + 1, T, q.h1, q.h2, q.nr, which, q.ro, q.S, q.theta);
-            NC_CHECK_LAUNCH();
-            ctx.launches++;
-            read_scalars(ctx, q.ro, sizeof(RitzOut), &rr);
         }
+        const RitzOut rr = lane.wait();
         const double anorm = std::max(std::fabs(rr.theta), eps23);
         last_ratio = rr.res / (tol_eff * anorm);
         if (rr.res <= tol_eff * anorm || j + 1 >= orth_dim) {

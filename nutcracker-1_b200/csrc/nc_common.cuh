@@ -132,6 +132,7 @@ struct Context {
     // projected problem of one Lanczos step beside the next step's product.
     cudaStream_t ritz_stream = nullptr;
     cudaEvent_t ritz_ready = nullptr, ritz_done = nullptr;
+    unsigned ritz_ticket = 0;   // marks the results of this thread's projected problems
     Context();
     ~Context();
     static Context& get();   // thread-local default context
