@@ -32,8 +32,13 @@ constexpr int RB = 296;       // 2 x 148 SMs
 constexpr int KC = 8;         // vectors per multi-dot chunk
 constexpr int MAXM = 128;     // largest multi-dot / multi-axpy width
 
-__global__ void multi_dot_partial(long long n, int k, const cplx* __restrict__ V,
-                                  const cplx* __restrict__ w, cplx* __restrict__ part) {
+// h = V^H w as block sums in `part`.  FUSED (one chunk of vectors): the last
+// block adds them as multi_dot_final does, so a filter through a few vectors is
+// one launch less; on a site of a few thousand elements a launch is all it costs.
+template <bool FUSED>
+__global__ void __launch_bounds__(RT) multi_dot_partial(long long n, int k, const cplx* __restrict__ V,
+                                                        const cplx* __restrict__ w, cplx* __restrict__ part,
+                                                        unsigned* __restrict__ counter, cplx* __restrict__ h) {
     // part[(chunk*KC + i) * gridDim.x + block]
     __shared__ double sr[KC][RT / 32], si[KC][RT / 32];
     const int c0 = blockIdx.y * KC;
@@ -71,6 +76,32 @@ __global__ void multi_dot_partial(long long n, int k, const cplx* __restrict__ V
             for (int q = 0; q < RT / 32; ++q) { r += sr[i][q]; im += si[i][q]; }
             part[(size_t)(c0 + i) * gridDim.x + blockIdx.x] = cmake(r, im);
         }
+    }
+    if constexpr (FUSED) {
+        __shared__ double tr[RT], ti[RT];
+        __shared__ bool last;
+        if (threadIdx.x < KC) __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        for (int i = 0; i < k; ++i) {
+            double r = 0, im = 0;
+            for (int b = threadIdx.x; b < (int)gridDim.x; b += RT) {
+                const cplx p = __ldcg(&part[(size_t)i * gridDim.x + b]);
+                r += p.x; im += p.y;
+            }
+            tr[threadIdx.x] = r; ti[threadIdx.x] = im;
+            __syncthreads();
+            for (int s = RT / 2; s > 0; s >>= 1) {
+                if ((int)threadIdx.x < s) { tr[threadIdx.x] += tr[threadIdx.x + s]; ti[threadIdx.x] += ti[threadIdx.x + s]; }
+                __syncthreads();
+            }
+            if (threadIdx.x == 0) h[i] = cmake(tr[0], ti[0]);
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) *counter = 0;
     }
 }
 
@@ -403,7 +434,13 @@ void multi_dotc(Context& ctx, long long n, int k, const cplx* V, const cplx* w, 
     int nb = (int)std::min<long long>(RB, std::max<long long>(1, (n + RT - 1) / RT));
     cplx* part = ctx.arena.alloc_n<cplx>((size_t)nb * ((k + KC - 1) / KC) * KC);
     dim3 grid(nb, (k + KC - 1) / KC);
-    multi_dot_partial<<<grid, RT, 0, ctx.stream>>>(n, k, V, w, part);
+    if (k <= KC) {   // the last block's sums take their turn, so only a few vectors
+        multi_dot_partial<true><<<grid, RT, 0, ctx.stream>>>(n, k, V, w, part, ctx.reduction_counter(), h);
+        NC_CHECK_LAUNCH();
+        ctx.launches++;
+        return;
+    }
+    multi_dot_partial<false><<<grid, RT, 0, ctx.stream>>>(n, k, V, w, part, nullptr, nullptr);
     NC_CHECK_LAUNCH();
     multi_dot_final<<<k, RT, 0, ctx.stream>>>(nb, part, h);
     NC_CHECK_LAUNCH();
