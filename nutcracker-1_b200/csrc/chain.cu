@@ -756,21 +756,29 @@ struct Chain {
     // Device bytes a chain of this operator needs at bond dimension
     // `bandwidth` for `levels` levels: the buffers allocate_for_bonds and the
     // projector sites hold, plus the solver's arena peak (Lanczos basis,
-    // H_eff scratch, the precision form's tensor-core operands) and the gauge
-    // moves' QR plans, with a 25% margin.
+    // H_eff scratch, the residue products' or the precision form's tensor-core
+    // operands) and the gauge moves' QR plans, with a 25% margin.
     static uint64_t footprint_bytes(const std::vector<int>& d, const std::vector<int>& cl, const std::vector<int>& cr,
                                     int bandwidth, int levels, int krylov, int precision) {
         const int n = (int)d.size();
         const int b = std::min(bandwidth, maximum_bandwidth_dimension(d));
         const std::vector<int> bonds = bandwidth_sequence(std::max(1, b), d);
-        double elems = 0, maxs = 1, maxenv = 1;
+        double elems = 0, maxs = 1, maxenv = 1, residue = 0;
         for (int i = 0; i < n; ++i) {
             const double site = (double)bonds[i] * bonds[i + 1] * d[i];
             maxs = std::max(maxs, site);
             const double env = (double)bonds[i] * bonds[i] * cl[i] + (double)bonds[i + 1] * bonds[i + 1] * cr[i];
             maxenv = std::max(maxenv, env);
             elems += env;
+            const long long bl = bonds[i], br = bonds[i + 1];      // H_eff's and the environment updates' GEMMs
+            for (const double bytes : {residue_scratch_bytes(br * d[i], bl * cl[i], bl),
+                                       residue_scratch_bytes(br, bl * d[i], br * cr[i]),
+                                       residue_scratch_bytes(br * cr[i], br, bl * d[i]),
+                                       residue_scratch_bytes(bl * d[i], br * cr[i], br),
+                                       residue_scratch_bytes(bl * cl[i], bl, br * d[i])})
+                residue = std::max(residue, bytes);
         }
+        elems += residue / sizeof(cplx);
         elems += (n + 2) * maxs;                                   // sites and spares
         const int np = std::max(0, levels - 1);
         for (int i = 0; i < n; ++i)                                // projector sites and overlap environments

@@ -187,6 +187,9 @@ struct ResMatrix {
 };
 // Whether an M x N x K complex product is faster through residues than on the DMMA pipe.
 bool residue_gemm_pays(long long M, long long N, long long K);
+// Scratch of one such product: 45 bytes an operand element, 30 an element of C
+// (none where residue_gemm_pays says no).
+double residue_scratch_bytes(long long M, long long N, long long K);
 // C(m,n) = sum_k A(m,k) B(n,k) to C[(m % I) + (m / I) * sI + n * sn] (scratch
 // from ctx.scratch()).
 void residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b, cplx* C, int I, long long sI,

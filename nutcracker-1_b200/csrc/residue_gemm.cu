@@ -691,6 +691,12 @@ void residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b, cplx*
     });
 }
 
+double residue_scratch_bytes(long long M, long long N, long long K) {
+    if (!residue_gemm_pays(M, N, K)) return 0;
+    const double rows = (double)((M + TM - 1) / TM * TM), cols = (double)((N + TN - 1) / TN * TN);
+    return 3.0 * NL * (double)(M + N) * padded_k((int)K) + 2.0 * NL * rows * cols;
+}
+
 void device_check(Context& ctx) {
     if (!ctx.check_pending) return;
     ctx.check_pending = false;
