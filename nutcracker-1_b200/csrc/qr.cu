@@ -548,7 +548,7 @@ cluster_block_qr_kernel(int mp, int nb, int rows_per_cta, cplx* __restrict__ A, 
 // on the FP64 tensor pipe (M = 8 reflectors or columns fits its m8n8k4 shape),
 // with V^H P summed over the CTAs by column slices once per sub-block.  v_c^H v_i for i < c
 // comes out of the column's own sums (they run over all eight columns), so it
-// costs nothing.  B200, one 2048 x 64 block: 212 -> SUBUS us.
+// costs nothing.  B200, one 2048 x 64 block: 212 -> 171 us.
 //
 // The one-block shapes (n <= 64) keep the kernel above: their results stay what
 // they were bit for bit (a chain's edge sites turn rounding into the phase of
