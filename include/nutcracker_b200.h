@@ -42,14 +42,15 @@ const char* nc_version(void);
 int nc_set_stream(void* stream);
 /* Go back to the library's own non-blocking stream (the initial state). */
 int nc_use_own_stream(void);
-/* Wait for this thread's stream.  Returns a status code. */
+/* Wait for this thread's stream.  Returns a status code: NC_ERR_TIMEOUT when
+   a bounded device wait of the work before it ran out. */
 int nc_synchronize(void);
 /* Start timing every complex GEMM of at least `min_flops` algorithmic flops
    with CUDA events on this thread's stream. */
 int nc_profile_begin(double min_flops);
-/* Stop timing; report the number of timed FP64 complex GEMMs, their summed
-   device time (ms) and summed algorithmic flops (8*M*N*K per complex
-   product). */
+/* Stop timing; report the number of timed FP64 complex GEMMs (on the DMMA
+   pipe or through residues, with their conversions), their summed device time
+   (ms) and summed algorithmic flops (8*M*N*K per complex product). */
 int nc_profile_end(uint64_t* launches, double* total_ms, double* total_flops);
 /* Without stopping: the same totals for one kind of timed GEMM, kind 0 =
    FP64 complex GEMM, kind 1 = tcgen05 3xTF32 GEMM (flops counted as the
