@@ -218,6 +218,7 @@ void launch_ops(const ZGemmParams& p, cudaStream_t s) {
     // output does not depend on the tile, so neither do the results.
     const long long z = (long long)p.batch * p.nsplit;
     auto load = [&](int bm, int bn, double w) {
+        if (ceil_div(p.M, bm) > 65535) return 1e30;   // the grid's y extent (a restart's basis has M up to millions)
         const long long t = (long long)ceil_div(p.M, bm) * ceil_div(p.N, bn) * z;
         return (double)((t + 147) / 148) * bm * bn * w;
     };
