@@ -589,19 +589,30 @@ CUtensorMap make_map8(const uint8_t* ptr, int Kp, int rows, int rows_p, int box_
     return m;
 }
 
+int padded_k(int K) { return (K + 63) / 64 * 64; }
+// Residue planes of both operands and the residues of C.
+double scratch_bytes(long long M, long long N, long long K) {
+    const double rows = (double)((M + TM - 1) / TM * TM), cols = (double)((N + TN - 1) / TN * TN);
+    return 3.0 * NL * (double)(M + N) * padded_k((int)K) + 2.0 * NL * rows * cols;
+}
+constexpr double kMaxScratch = 16.0 * (1 << 30);
+
 }  // namespace
 
 // Measured on a B200, one H_eff product of a Heisenberg site (two GEMMs and
 // the mix), DMMA route against this one: chi = 192 80 / 116 us, 224 109 / 129,
 // 256 200 / 135, 320 352 / 173, 512 1020 / 345, 1024 5750 / 1362.  The
 // crossing lies near 2^27 complex multiplications a GEMM; below one tile of
-// rows or half a tile of columns the padding costs more.  Error against
+// rows or half a tile of columns the padding costs more.  Products whose
+// residues would take more than 16 GB (several times the operands) or whose
+// columns exceed the CRT's grid stay on the DMMA pipe.  Error against
 // extended precision (2-norm, chi = 256 / 1024): DMMA 4.3e-16 / 2.2e-15, this
 // route 1.4e-16 / 2.9e-16.  The error is relative to the norms of the rows of
 // A and the columns of B: an output far below |a_m| |b_n| can be off by more
 // than its own rounding.
 bool residue_gemm_pays(long long M, long long N, long long K) {
-    return M >= TM && N >= TN / 2 && K >= 64 && K <= kMaxK && M * N * K >= (1LL << 27);
+    return M >= TM && N >= TN / 2 && K >= 64 && K <= kMaxK && M * N * K >= (1LL << 27) && N <= 4 * 65535 &&
+           scratch_bytes(M, N, K) <= kMaxScratch;
 }
 
 namespace {
@@ -611,7 +622,6 @@ struct ResOperand {
     int rows, K, Kp;
 };
 
-int padded_k(int K) { return (K + 63) / 64 * 64; }
 
 // Residue planes and row scales of both operands (scratch of the caller's frame).
 void residue_convert(Context& ctx, const ResMatrix* const (&src)[2], ResOperand (&out)[2]) {
@@ -692,9 +702,7 @@ void residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b, cplx*
 }
 
 double residue_scratch_bytes(long long M, long long N, long long K) {
-    if (!residue_gemm_pays(M, N, K)) return 0;
-    const double rows = (double)((M + TM - 1) / TM * TM), cols = (double)((N + TN - 1) / TN * TN);
-    return 3.0 * NL * (double)(M + N) * padded_k((int)K) + 2.0 * NL * rows * cols;
+    return residue_gemm_pays(M, N, K) ? scratch_bytes(M, N, K) : 0;
 }
 
 void device_check(Context& ctx) {
