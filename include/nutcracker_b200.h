@@ -61,7 +61,16 @@ int nc_profile_query(int kind, uint64_t* launches, double* total_ms, double* tot
    (the strategy-3 `operate_on` of core.f95:2529-2556 without projectors):
    L (bl,bl,cl), R (br,br,cr), x and y (br,bl,d), W (d,d,nnz), idx (2,nnz)
    1-based, all in device memory.  Scratch comes from the library's device
-   arena.  Asynchronous on this thread's stream; returns a status code. */
+   arena.  Asynchronous on this thread's stream; returns a status code.
+
+   FP64 contractions of at least 3 * 2^28 complex multiplications (here, in
+   the environment updates and in the gauge moves) run in integers on the int8
+   tensor cores when the integers hold the operands: components above 2^-24 of
+   their row's (column's) norm keep all their bits, and no more than one
+   component in 2^15 may lose any (to 2^-77 of the norm).  Decided on the
+   device from the operands; others, and operands with an infinity or a NaN,
+   are multiplied in FP64 as smaller ones are.  Scratch for the integers: 60
+   bytes an operand element and 40 an output element. */
 int nc_heff_apply_dev(uint32_t bl, uint32_t br, uint32_t cl, uint32_t cr, uint32_t d, uint32_t nnz,
                       const uint32_t* idx_dev, const void* W_dev, const void* L_dev,
                       const void* R_dev, const void* x_dev, void* y_dev);
@@ -120,7 +129,8 @@ int nc_test_tc32_wait(uint64_t wait_ns, int skip_first_load);
    that loads the library holds until exit.  A call needs
    16*(br*bl*cl*d + br*cr*bl*d) bytes of it; larger calls return an error
    and launch nothing.  Work is enqueued on `stream` (a cudaStream_t, NULL =
-   legacy default stream).  The first call on each device looks the array's
+   legacy default stream).  The contractions are always FP64 ones, in one
+   pass over K.  The first call on each device looks the array's
    device address up (cudaGetSymbolAddress); make it before any stream
    capture.  All calls share the array and each rewrites it completely, so
    nothing needs clearing, but calls that overlap on the GPU race: order them

@@ -276,7 +276,7 @@ void mix_right(Context& ctx, int bl, int br, const MpoSite& op, const cplx* Y, c
     ctx.launches++;
 }
 
-// An operand of residue_product: row i = (i % I, i / I) at strides (si, sI), K index at stride sk.
+// An operand of zproduct: row i = (i % I, i / I) at strides (si, sI), K index at stride sk.
 ResMatrix res_matrix(const cplx* X, int rows, int K, long long si, long long sk, bool conj = false, int I = 0,
                      long long sI = 0) {
     ResMatrix m;
@@ -288,16 +288,12 @@ ResMatrix res_matrix(const cplx* X, int rows, int K, long long si, long long sk,
 // Step A of H_eff / sos_left: T(r,j,k1,a) = sum_i psi(r,i,a) L(i,j,k1)
 void stage_a(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L, const cplx* psi,
              cplx* T) {
-    if (residue_gemm_pays((long long)br * op.d, (long long)bl * op.cl, bl)) {
-        // the d products share L: rows (r, a) of one product
-        residue_product(ctx, res_matrix(psi, br * op.d, bl, 1, br, false, br, (long long)br * bl),
-                        res_matrix(L, bl * op.cl, bl, bl, 1), T, br, (long long)br * bl * op.cl, br);
-        return;
-    }
     ZGemmParams p = zgemm_params(OP_N, OP_N, br, bl * op.cl, bl, psi, br, L, bl, T, br);
     p.batch = op.d;
     p.sA0 = (long long)br * bl; p.sB0 = 0; p.sC0 = (long long)br * bl * op.cl;
-    zgemm(p, ctx);
+    // the d products share L: rows (r, a) of one product
+    zproduct(ctx, p, res_matrix(psi, br * op.d, bl, 1, br, false, br, (long long)br * bl),
+             res_matrix(L, bl * op.cl, bl, bl, 1), br, (long long)br * bl * op.cl, br);
 }
 
 }  // namespace
@@ -313,17 +309,13 @@ void heff_apply(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L, 
     cplx* U = ws + (size_t)br * bl * op.cl * op.d;
     stage_a(ctx, bl, br, op, L, x, T);
     mix_left(ctx, bl, br, op, T, U);
-    if (residue_gemm_pays(br, (long long)bl * op.d, (long long)br * op.cr)) {
-        // the d products share Rhat: columns (j, b) of one product
-        residue_product(ctx, res_matrix(R, br, br * op.cr, 1, br),
-                        res_matrix(U, bl * op.d, br * op.cr, (long long)br * op.cr, 1), y, br, 0, br);
-        return;
-    }
     // out_b = Rhat (br x br*cr) * Uhat_b (br*cr x bl)
     ZGemmParams p = zgemm_params(OP_N, OP_N, br, bl, br * op.cr, R, br, U, (long long)br * op.cr, y, br);
     p.batch = op.d;
     p.sA0 = 0; p.sB0 = (long long)br * op.cr * bl; p.sC0 = (long long)br * bl;
-    zgemm(p, ctx);
+    // the d products share Rhat: columns (j, b) of one product
+    zproduct(ctx, p, res_matrix(R, br, br * op.cr, 1, br), res_matrix(U, bl * op.d, br * op.cr, (long long)br * op.cr, 1),
+             br, 0, br);
 }
 
 void heff_apply_stream(cudaStream_t s, int bl, int br, const MpoSite& op, const cplx* L, const cplx* R,
@@ -354,15 +346,11 @@ void sos_left(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L, co
     stage_a(ctx, bl, br, op, L, psi, T);
     mix_left(ctx, bl, br, op, T, U);
     // L'_{k2}(r,r'') = sum_{(j,b)} U(r,k2,j,b) conj(psi(r'',j,b))
-    if (residue_gemm_pays((long long)br * op.cr, br, (long long)bl * op.d)) {
-        residue_product(ctx, res_matrix(U, br * op.cr, bl * op.d, 1, (long long)br * op.cr),
-                        res_matrix(psi, br, bl * op.d, 1, br, true), Lnew, br, (long long)br * br, br);
-        return;
-    }
     ZGemmParams p = zgemm_params(OP_N, OP_C, br, br, bl * op.d, U, (long long)br * op.cr, psi, br, Lnew, br);
     p.batch = op.cr;
     p.sA0 = br; p.sB0 = 0; p.sC0 = (long long)br * br;
-    zgemm(p, ctx);
+    zproduct(ctx, p, res_matrix(U, br * op.cr, bl * op.d, 1, (long long)br * op.cr),
+             res_matrix(psi, br, bl * op.d, 1, br, true), br, (long long)br * br, br);
 }
 
 void sos_right(Context& ctx, int bl, int br, const MpoSite& op, const cplx* R, const cplx* psi,
@@ -374,25 +362,18 @@ void sos_right(Context& ctx, int bl, int br, const MpoSite& op, const cplx* R, c
     cplx* Z = ctx.arena.alloc_n<cplx>((size_t)bl * br * d * op.cl);
     cplx* Pp = ctx.arena.alloc_n<cplx>((size_t)br * d * bl);
     // Y(x,b,r,k2) = sum_r'' conj(psi(r'',x,b)) R(r'',r,k2)
-    if (residue_gemm_pays((long long)bl * d, (long long)br * op.cr, br))
-        residue_product(ctx, res_matrix(psi, bl * d, br, br, 1, true), res_matrix(R, br * op.cr, br, br, 1), Y, bl * d, 0,
-                        (long long)bl * d);
-    else
-        zgemm(zgemm_params(OP_C, OP_N, bl * d, br * op.cr, br, psi, br, R, br, Y, (long long)bl * d), ctx);
+    zproduct(ctx, zgemm_params(OP_C, OP_N, bl * d, br * op.cr, br, psi, br, R, br, Y, (long long)bl * d),
+             res_matrix(psi, bl * d, br, br, 1, true), res_matrix(R, br * op.cr, br, br, 1), bl * d, 0, (long long)bl * d);
     mix_right(ctx, bl, br, op, Y, Z);
     // Pp(r,a,y) = psi(r,y,a)
     const int perm[3] = {0, 2, 1};
     permute3(ctx, psi, br, bl, d, perm, false, Pp);
     // R'_{k1} = Z_{k1} (bl x br*d) * Pp (br*d x bl)
-    if (residue_gemm_pays((long long)bl * op.cl, bl, (long long)br * d)) {
-        residue_product(ctx, res_matrix(Z, bl * op.cl, br * d, 1, bl, false, bl, (long long)bl * br * d),
-                        res_matrix(Pp, bl, br * d, (long long)br * d, 1), Rnew, bl, (long long)bl * bl, bl);
-        return;
-    }
     ZGemmParams q = zgemm_params(OP_N, OP_N, bl, bl, br * d, Z, bl, Pp, (long long)br * d, Rnew, bl);
     q.batch = op.cl;
     q.sA0 = (long long)bl * br * d; q.sB0 = 0; q.sC0 = (long long)bl * bl;
-    zgemm(q, ctx);
+    zproduct(ctx, q, res_matrix(Z, bl * op.cl, br * d, 1, bl, false, bl, (long long)bl * br * d),
+             res_matrix(Pp, bl, br * d, (long long)br * d, 1), bl, (long long)bl * bl, bl);
 }
 
 void vs_left(Context& ctx, int blo, int bro, int bln, int brn, int d, const cplx* Lov,

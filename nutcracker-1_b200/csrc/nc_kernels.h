@@ -35,6 +35,17 @@ void profile_launch(Context& ctx, double flops, int kind, F&& launch) {
 
 enum Op { OP_N = 0, OP_T = 1, OP_C = 2 };
 
+// Which of two products of the same operands runs (residue_gemm.cu): the one
+// through residues while no operand has more rounded components than its limit,
+// else the FP64 one.  Decided on the device, by kernels that return at once.
+struct ResidueGate {
+    const unsigned long long* rounded = nullptr;   // per operand
+    unsigned long long limit[2] = {0, 0};
+};
+__device__ __forceinline__ bool residues_hold(const ResidueGate& g) {
+    return g.rounded[0] <= g.limit[0] && g.rounded[1] <= g.limit[1];
+}
+
 struct ZGemmParams {
     int opA, opB;
     int M, N, K;
@@ -45,6 +56,7 @@ struct ZGemmParams {
     cplx alpha, beta;
     int kchunk, nsplit;  // split-K (set by zgemm(p, ctx); 0/1 = none)
     cplx* ws;            // split-K partials
+    ResidueGate gate;    // with `rounded`: runs only where the residues do not hold the operands
 };
 
 ZGemmParams zgemm_params(int opA, int opB, int M, int N, int K, const cplx* A, long long lda,
@@ -53,6 +65,8 @@ ZGemmParams zgemm_params(int opA, int opB, int M, int N, int K, const cplx* A, l
 void zgemm(const ZGemmParams& p, cudaStream_t s);
 // Launch with automatic split-K when the tile grid is small (workspace from ctx.arena).
 void zgemm(const ZGemmParams& p, Context& ctx);
+// The same without an entry in nc_profile_*.
+void zgemm_untimed(const ZGemmParams& p, Context& ctx);
 void scale_strided(const ZGemmParams& p, cudaStream_t s);
 
 // One MPO site on the device: W (d,d,nnz) column-major, idx (2,nnz) 1-based.
@@ -187,13 +201,14 @@ struct ResMatrix {
 };
 // Whether an M x N x K complex product is faster through residues than on the DMMA pipe.
 bool residue_gemm_pays(long long M, long long N, long long K);
-// Scratch of one such product: 45 bytes an operand element, 30 an element of C
+// Scratch of one such product: 60 bytes an operand element, 40 an element of C
 // (none where residue_gemm_pays says no).
 double residue_scratch_bytes(long long M, long long N, long long K);
-// C(m,n) = sum_k A(m,k) B(n,k) to C[(m % I) + (m / I) * sI + n * sn] (scratch
-// from ctx.scratch()).
-void residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b, cplx* C, int I, long long sI,
-                     long long sn);
+// zgemm(p) (alpha 1, beta 0), written a second time as C(m,n) = sum_k A(m,k)
+// B(n,k) to p.C[(m % I) + (m / I) * sI + n * sn]: through residues where that
+// pays and holds the operands (scratch from ctx.scratch()).
+void zproduct(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResMatrix& b, int I, long long sI,
+              long long sn);
 // Synchronises ctx.stream and raises NC_ERR_TIMEOUT if a bounded wait of a
 // residue GEMM or cluster QR launched since the last check expired; returns at
 // once when none was.

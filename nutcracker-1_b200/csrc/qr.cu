@@ -1183,20 +1183,12 @@ void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int 
     if (!Q) return;
     // Z = T V_1^H, Q = I - V Z
     ResMatrix a, b;
-    if (residue_gemm_pays(n, n, n)) {
-        a.X = T; a.rows = n; a.K = n; a.si = 1; a.sk = n; a.I = n;
-        b.X = V; b.rows = n; b.K = n; b.si = 1; b.sk = m; b.I = n; b.conj = 1;
-        residue_product(ctx, a, b, Z, n, 0, n);
-    } else {
-        zgemm(zgemm_params(OP_N, OP_C, n, n, n, T, n, V, m, Z, n), ctx);
-    }
-    if (residue_gemm_pays(m, n, n)) {
-        a.X = V; a.rows = m; a.K = n; a.si = 1; a.sk = m; a.I = m; a.conj = 0;
-        b.X = Z; b.rows = n; b.K = n; b.si = n; b.sk = 1; b.I = n; b.conj = 0;
-        residue_product(ctx, a, b, Q, m, 0, m);
-    } else {
-        zgemm(zgemm_params(OP_N, OP_N, m, n, n, V, m, Z, n, Q, m), ctx);
-    }
+    a.X = T; a.rows = n; a.K = n; a.si = 1; a.sk = n; a.I = n;
+    b.X = V; b.rows = n; b.K = n; b.si = 1; b.sk = m; b.I = n; b.conj = 1;
+    zproduct(ctx, zgemm_params(OP_N, OP_C, n, n, n, T, n, V, m, Z, n), a, b, n, 0, n);
+    a.X = V; a.rows = m; a.K = n; a.si = 1; a.sk = m; a.I = m; a.conj = 0;
+    b.X = Z; b.rows = n; b.K = n; b.si = n; b.sk = 1; b.I = n; b.conj = 0;
+    zproduct(ctx, zgemm_params(OP_N, OP_N, m, n, n, V, m, Z, n, Q, m), a, b, m, 0, m);
     one_minus_kernel<<<gsz((long long)m * n), 256, 0, ctx.stream>>>(m, n, Q);
     NC_CHECK_LAUNCH();
     ctx.launches++;
@@ -1361,7 +1353,7 @@ void qr_run(Context& ctx, QrPlan& P) {
 static void absorb_factor(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResMatrix& b, int I,
                           long long sI, long long sn, const AbsorbAsync* as) {
     if (residue_gemm_pays(a.rows, b.rows, a.K)) {
-        residue_product(ctx, a, b, p.C, I, sI, sn);
+        zproduct(ctx, p, a, b, I, sI, sn);
         if (as) NC_CUDA(cudaEventRecord(as->done, ctx.stream));
         return;
     }
