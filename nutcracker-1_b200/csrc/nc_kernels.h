@@ -55,6 +55,7 @@ struct ZGemmParams {
     int nb0, batch;   // batch index b = b0 + nb0*b1; nb0 = 0: one level (b0 = b)
     cplx alpha, beta;
     int kchunk, nsplit;  // split-K (set by zgemm(p, ctx); 0/1 = none)
+    int chain = 0;       // longest K summed in one chain by zgemm(p, ctx), a multiple of 16; 0: any
     cplx* ws;            // split-K partials
     ResidueGate gate;    // with `rounded`: runs only where the residues do not hold the operands
 };

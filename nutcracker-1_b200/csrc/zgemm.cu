@@ -269,6 +269,7 @@ void zgemm_untimed(const ZGemmParams& p_in, Context& ctx) {
         nsplit = (int)std::min<long long>((2 * 148 + tiles - 1) / tiles, p.K / 128);
         nsplit = std::max(1, std::min(nsplit, 32));
     }
+    if (p.chain > 0) nsplit = std::max(nsplit, (p.K + p.chain - 1) / p.chain);
     if (nsplit <= 1) {
         zgemm(p, ctx.stream);
         ctx.launches++;
