@@ -43,7 +43,8 @@ int nc_set_stream(void* stream);
 /* Go back to the library's own non-blocking stream (the initial state). */
 int nc_use_own_stream(void);
 /* Wait for this thread's stream.  Returns a status code: NC_ERR_TIMEOUT when
-   a bounded device wait of the work before it ran out. */
+   a bounded device wait of this thread's work before it ran out (reported
+   once, by the first call of the thread that waits for its work). */
 int nc_synchronize(void);
 /* Start timing every complex GEMM of at least `min_flops` algorithmic flops
    with CUDA events on this thread's stream. */
@@ -111,14 +112,17 @@ int nc_gauge_move_dev(int direction, uint32_t bl, uint32_t bm, uint32_t br, uint
 int nc_tc_zgemm_dev(uint32_t M, uint32_t N, uint32_t K, const void* A_dev, const void* B_dev,
                     void* C_dev, int three);
 
-/* No counterpart in the reference; for tests of the failure path.  Sets
-   the time limit of every mbarrier wait in the tcgen05 GEMM (default 2 s,
-   here in nanoseconds, at least 1000) and, when skip_first_load is nonzero,
-   makes tile (0,0,0) of the following GEMMs leave its first K stage
-   unloaded, so that a wait runs out: the kernel then stops issuing, leaves
-   through its final barrier and frees its tensor memory, and the host call
-   reports NC_ERR_TIMEOUT.  Process-wide; restore (2000000000, 0) after use.
-   Returns a status code. */
+/* No counterpart in the reference; for tests of the failure paths.  Sets the
+   time limit of every bounded device wait of this thread's kernels (default
+   2 s, here in nanoseconds, at least 1000): the tcgen05 GEMM's and the residue
+   GEMM's pipelines and the exchange between the CTAs of a QR panel.  `mute` is
+   the sum of 1 (tcgen05 GEMM: tile (0,0,0) leaves its first K stage unloaded)
+   and 2 (residue GEMM: CTA 0 leaves its first K stage unloaded): a wait of
+   that kernel then runs out, it returns, and the next call of this thread
+   that waits for its work reports NC_ERR_TIMEOUT.  Restore (2000000000, 0)
+   after use.  Waits for this thread's stream; returns a status code. */
+int nc_test_device_wait(uint64_t wait_ns, uint32_t mute);
+/* The same for the tcgen05 GEMM: mute is 1 when skip_first_load is nonzero. */
 int nc_test_tc32_wait(uint64_t wait_ns, int skip_first_load);
 
 /* No counterpart in the reference.  The same H_eff product as

@@ -178,8 +178,7 @@ int nc_profile_query(int kind, uint64_t* launches, double* total_ms, double* tot
 
 int nc_synchronize(void) {
     NC_ABI_BEGIN
-    NC_CUDA(cudaStreamSynchronize(Context::get().stream));
-    device_check(Context::get());
+    Context::get().settle();
     NC_ABI_END
     return g_status;
 }
@@ -212,7 +211,7 @@ int nc_heff_apply_mixed_dev(uint32_t bl, uint32_t br, uint32_t cl, uint32_t cr, 
     MixedHeff h;
     mixed_heff_prepare(ctx, bl, br, op, (const cplx*)L_dev, (const cplx*)R_dev, buf, &h);
     heff_apply_mixed(ctx, h, (const cplx*)x_dev, (cplx*)y_dev);
-    tc_check(ctx);
+    ctx.settle();
     NC_ABI_END
     return g_status;
 }
@@ -236,7 +235,7 @@ int nc_env_update_dev(int side, int mixed, uint32_t bl, uint32_t br, uint32_t cl
         if (mixed) sos_right_mixed(ctx, bl, br, op, env, psi, out);
         else sos_right(ctx, bl, br, op, env, psi, out);
     }
-    if (mixed) tc_check(ctx);
+    if (mixed) ctx.settle();
     NC_ABI_END
     return g_status;
 }
@@ -250,9 +249,19 @@ int nc_tc_zgemm_dev(uint32_t M, uint32_t N, uint32_t K, const void* A_dev, const
     return g_status;
 }
 
+int nc_test_device_wait(uint64_t wait_ns, uint32_t mute) {
+    NC_ABI_BEGIN
+    NC_ARG(wait_ns >= 1000, "the wait limit must be at least 1 microsecond");
+    NC_ARG(mute < (1u << WATCH_KINDS), "unknown kind of wait");
+    Context::get().set_watch((unsigned long long)wait_ns, mute);
+    NC_ABI_END
+    return g_status;
+}
+
 int nc_test_tc32_wait(uint64_t wait_ns, int skip_first_load) {
     NC_ABI_BEGIN
-    tc_test_fault((unsigned long long)wait_ns, skip_first_load);
+    NC_ARG(wait_ns >= 1000, "tc32 wait limit must be at least 1 microsecond");
+    Context::get().set_watch((unsigned long long)wait_ns, skip_first_load ? 1u << WATCH_TC32 : 0u);
     NC_ABI_END
     return g_status;
 }

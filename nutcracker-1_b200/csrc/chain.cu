@@ -562,11 +562,8 @@ struct Chain {
         while (cur + 1 < N) { move(+1); optimize_site(); }
         while (cur > 0) { move(-1); optimize_site(); }
         while (cur < start) { move(+1); optimize_site(); }
-        if (prec) {
-            tc_check(ctx);
-            stats.mixed_sweeps++;
-        }
-        device_check(ctx);
+        ctx.settle();
+        if (prec) stats.mixed_sweeps++;
         if (free_sweeps > 0) --free_sweeps;
         stats.sweeps++;
         emit(NC_SIGNAL_SWEEP_PERFORMED, (int64_t)stats.sweeps);   // chain.cpp:162

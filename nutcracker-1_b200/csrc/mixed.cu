@@ -507,7 +507,7 @@ void tc_zgemm(Context& ctx, int M, int N, int K, const cplx* A, const cplx* B, c
     g.M = M; g.Nr = 2 * N; g.Kr = 2 * K; g.batch = 1;
     g.C = C; g.sm = 1; g.sn = M; g.sz = 0; g.c_fp64 = true; g.three = three;
     tc_gemm(ctx, g);
-    tc_check(ctx);
+    ctx.settle();
 }
 
 }  // namespace nc

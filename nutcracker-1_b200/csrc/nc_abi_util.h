@@ -43,10 +43,7 @@ struct HostStage {
         if (n == 0) return;
         NC_CUDA(cudaMemcpyAsync(host, dev, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx.stream));
     }
-    void sync() {
-        NC_CUDA(cudaStreamSynchronize(ctx.stream));
-        device_check(ctx);
-    }
+    void sync() { ctx.settle(); }
 
     MpoSite mpo(uint32_t d, uint32_t cl, uint32_t cr, uint32_t nnz, const uint32_t* idx,
                 const nc_complex* W) {

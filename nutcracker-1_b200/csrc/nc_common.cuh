@@ -88,6 +88,26 @@ struct ArenaFrame {
     ~ArenaFrame() { a.release(m); }
 };
 
+// The bounded waits of a context's kernels, in device memory: their time limit,
+// and where an expired one leaves its mark (one pinned host word a kind, so that
+// the host sees it after any synchronisation without a copy).  `mute` (bit
+// 1 << kind) is for tests: such a kernel withholds one arrival, so that a wait
+// runs out.
+enum WatchKind { WATCH_TC32 = 0, WATCH_RESIDUE = 1, WATCH_QR = 2, WATCH_KINDS = 3 };
+struct DeviceWatch {
+    unsigned long long limit_ns;
+    unsigned mute;
+    volatile unsigned* expired;
+};
+__device__ __forceinline__ void watch_expired(const DeviceWatch* w, int kind) {
+    w->expired[kind] = 1u;
+    __threadfence_system();
+}
+// The limit of a wait that has lasted `elapsed` ns, 0 while that is too short to ask.
+__device__ __forceinline__ bool watch_over(const DeviceWatch* w, unsigned long long elapsed) {
+    return elapsed > 1000ull && elapsed > *reinterpret_cast<const volatile unsigned long long*>(&w->limit_ns);
+}
+
 // Per-host-thread execution context: stream, arena and small pinned buffers.
 struct Context {
     int device = 0;
@@ -98,8 +118,12 @@ struct Context {
     size_t pinned_bytes = 0;
     uint64_t launches = 0;   // kernels launched by this library on this context
     int krylov_dim = 24;     // Lanczos basis size before a restart
-    // a kernel with bounded waits (residue GEMM, cluster QR) was launched since the last device_check
-    bool check_pending = false;
+    // Bounded waits of this context's kernels, on whatever stream they run.
+    DeviceWatch* watch = nullptr;       // device memory
+    volatile unsigned* expired = nullptr;   // its marks, pinned
+    void set_watch(unsigned long long limit_ns, unsigned mute);   // synchronises
+    // Raises NC_ERR_TIMEOUT, once, when a wait of work that has ended expired.
+    void raise_expired();
     // Gauge of the Level-0 norm_denorm_* / norm_for_* entry points: true
     // (default) = the reference's exact polar factor, false = the faster
     // Householder-QR gauge (the same state, a different site tensor).
@@ -128,6 +152,12 @@ struct Context {
     bool blocking_sync = false;
     cudaEvent_t sync_event = nullptr;
     void sync();
+    // Waits for the stream and answers for its work (raise_expired): every place
+    // that hands results to the host goes through it.
+    void settle() {
+        sync();
+        raise_expired();
+    }
     // Second stream of the site solver (created at its first use): the
     // projected problem of one Lanczos step beside the next step's product.
     cudaStream_t ritz_stream = nullptr;

@@ -161,8 +161,6 @@ int convert_vectors_to_reflectors_dev(Context& ctx, long long m, int n, cplx* A,
 // triangle of A; optional explicit Q (m x n) and R (n x n, zeros below,
 // conjugated if conjR).
 void householder_qr(Context& ctx, int m, int n, cplx* A, cplx* Q, cplx* R, bool conjR);
-// Whether a wait of the cluster QR has expired since the last call (for device_check).
-int qr_take_error();
 
 // ---- tcgen05 3xTF32 complex GEMM (tc32.cu) ---------------------------------
 // One operand of the real GEMM: rows x Kr floats, Kr contiguous, row stride
@@ -185,11 +183,6 @@ struct TcGemm {
     bool three = true;   // false: big x big only (one TF32 product)
 };
 void tc_gemm(Context& ctx, const TcGemm& g);
-// Synchronises ctx.stream; raises NC_ERR_TIMEOUT if a tc32 pipeline wait expired.
-void tc_check(Context& ctx);
-// Test hook: the limit of every tc32 mbarrier wait (ns) and the switch that
-// leaves the first K stage of tile (0,0,0) unloaded (its wait then runs out).
-void tc_test_fault(unsigned long long wait_ns, int skip_first_load);
 
 // ---- complex128 GEMM through residues on the int8 tensor cores (residue_gemm.cu)
 // One operand: row i, K index k at X[(i % I) * si + (i / I) * sI + k * sk]
@@ -210,10 +203,6 @@ double residue_scratch_bytes(long long M, long long N, long long K);
 // pays and holds the operands (scratch from ctx.scratch()).
 void zproduct(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResMatrix& b, int I, long long sI,
               long long sn);
-// Synchronises ctx.stream and raises NC_ERR_TIMEOUT if a bounded wait of a
-// residue GEMM or cluster QR launched since the last check expired; returns at
-// once when none was.
-void device_check(Context& ctx);
 
 // ---- precision form of the site products (mixed.cu) ------------------------
 // Tensor-core operands of one site's H_eff (environments expanded once per
@@ -240,7 +229,7 @@ void expectation_mixed(Context& ctx, const MixedHeff& h, const cplx* psi, cplx* 
 void sos_left_mixed(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L, const cplx* psi, cplx* Lnew);
 void sos_right_mixed(Context& ctx, int bl, int br, const MpoSite& op, const cplx* R, const cplx* psi, cplx* Rnew);
 // C (M x N) = A (M x K) B (K x N), column-major complex128, through tc_gemm;
-// three = false uses one TF32 product.  Synchronises and checks tc_check.
+// three = false uses one TF32 product.  Synchronises (Context::settle).
 void tc_zgemm(Context& ctx, int M, int N, int K, const cplx* A, const cplx* B, cplx* C, bool three);
 // Second stream for the neighbour's absorption of the gauge factor: the GEMM
 // waits on `ready` (recorded on ctx.stream after the QR), runs on `stream` and

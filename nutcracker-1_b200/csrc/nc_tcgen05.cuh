@@ -28,13 +28,13 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Bounded wait: false (and *error set) when the phase did not complete in `limit` ns.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned long long limit, int* error) {
+// Bounded wait: false (and the watch's mark set) when the phase did not complete in its limit.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const DeviceWatch* watch, int kind) {
     if (mbar_test(bar, parity)) return true;
     const unsigned long long t0 = gtimer();
     while (!mbar_test(bar, parity)) {
-        if (gtimer() - t0 > limit) {
-            atomicExch(error, 1);
+        if (watch_over(watch, gtimer() - t0)) {
+            watch_expired(watch, kind);
             return false;
         }
     }

@@ -575,8 +575,7 @@ struct SubSmem {
 // Remote stores whose arrival the receiver waits for on its own mbarrier
 // (st.async): a column needs one way through the cluster, not a cluster barrier
 // with its stores before it (2.9 -> 1.9 thousand cycles a column at 16 CTAs).
-// The wait is bounded by the global timer and reports through g_qr_error.
-__device__ int g_qr_error = 0;
+// The wait is bounded by the global timer and reports through the context's watch.
 __device__ __forceinline__ uint32_t remote(const void* p, int cta) {
     uint32_t r;
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(cta));
@@ -597,14 +596,14 @@ __device__ __forceinline__ bool arrived(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ void wait_sums(uint32_t bar, uint32_t parity, bool& alive) {
+__device__ __forceinline__ void wait_sums(uint32_t bar, uint32_t parity, bool& alive, const DeviceWatch* watch) {
     if (!alive || arrived(bar, parity)) return;
     unsigned long long t0, t1;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
     while (!arrived(bar, parity)) {
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-        if (t1 - t0 > 2000000000ull) {   // give up for good: every later wait returns at once
-            atomicExch(&g_qr_error, 1);
+        if (watch_over(watch, t1 - t0)) {   // give up for good: every later wait returns at once
+            watch_expired(watch, WATCH_QR);
             alive = false;
             return;
         }
@@ -631,7 +630,8 @@ __device__ __forceinline__ void t_column(SubSmem& s, int g, int lane) {
 
 __global__ void __launch_bounds__(CQ_T, 1)
 cluster_subblock_qr_kernel(int mp, int nb, int rows_per_cta, cplx* __restrict__ A, long long lda,
-                           cplx* __restrict__ V, long long ldv, cplx* __restrict__ tau_out) {
+                           cplx* __restrict__ V, long long ldv, cplx* __restrict__ tau_out,
+                           const DeviceWatch* __restrict__ watch) {
     extern __shared__ __align__(16) unsigned char sub_smem[];
     SubSmem& s = *reinterpret_cast<SubSmem*>(sub_smem);
     cg::cluster_group cluster = cg::this_cluster();
@@ -712,7 +712,7 @@ cluster_subblock_qr_kernel(int mp, int nb, int rows_per_cta, cplx* __restrict__ 
                 }
             }
             if (tid < 32 && jj > 0) t_column(s, jj - 1, lane);   // while the sums travel
-            wait_sums(bars + 8 * p, (uint32_t)(j >> 1) & 1u, alive);
+            wait_sums(bars + 8 * p, (uint32_t)(j >> 1) & 1u, alive, watch);
             // every thread: the totals of its column and of column jj, in a fixed tree
             const int src = lane & (span - 1);
             cplx Sc = src < 2 * C ? s.recv[p][c][src] : cmake(0, 0);
@@ -902,20 +902,6 @@ bool cluster_qr_probe() {
     return nclusters >= 1 && nsub >= 1;
 }
 
-}  // namespace
-
-int qr_take_error() {
-    int flag = 0;
-    NC_CUDA(cudaMemcpyFromSymbol(&flag, g_qr_error, sizeof(int)));
-    if (flag) {
-        const int zero = 0;
-        NC_CUDA(cudaMemcpyToSymbol(g_qr_error, &zero, sizeof(int)));
-    }
-    return flag;
-}
-
-namespace {
-
 bool cluster_qr_available() {
     static std::atomic<int> state[64];   // 0 unknown, 1 available, 2 not available
     int dev = 0;
@@ -947,8 +933,8 @@ void launch_cluster_block(Context& ctx, bool sub, int mp, int nb, cplx* A, long 
     cfg.numAttrs = 1;
     if (sub) {
         cfg.dynamicSmemBytes = sizeof(SubSmem);
-        NC_CUDA(cudaLaunchKernelEx(&cfg, cluster_subblock_qr_kernel, mp, nb, rows, A, lda, V, ldv, tau));
-        ctx.check_pending = true;
+        NC_CUDA(cudaLaunchKernelEx(&cfg, cluster_subblock_qr_kernel, mp, nb, rows, A, lda, V, ldv, tau,
+                                   static_cast<const DeviceWatch*>(ctx.watch)));
     } else {
         NC_CUDA(cudaLaunchKernelEx(&cfg, cluster_block_qr_kernel, mp, nb, rows, A, lda, V, ldv, tau));
     }
@@ -1222,6 +1208,7 @@ void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int 
 // input/output buffers and a private workspace arena, so the pointers baked
 // into the graph stay valid and are never shared with other work.
 struct QrPlan {
+    const Context* owner = nullptr;   // its graph reports expired waits to this context
     int m = 0, n = 0;
     bool conjR = false;
     Arena arena;
@@ -1256,8 +1243,9 @@ Context& side_context() {
 QrPlan& qr_plan(Context& ctx, int m, int n, bool conjR) {
     thread_local std::vector<std::unique_ptr<QrPlan>> plans;
     for (auto& p : plans)
-        if (p->m == m && p->n == n && p->conjR == conjR) return *p;
+        if (p->owner == &ctx && p->m == m && p->n == n && p->conjR == conjR) return *p;
     auto p = std::make_unique<QrPlan>();
+    p->owner = &ctx;
     p->m = m; p->n = n; p->conjR = conjR;
     p->X = p->arena.alloc_n<cplx>((size_t)m * n);
     p->Q = p->arena.alloc_n<cplx>((size_t)m * n);
@@ -1295,7 +1283,6 @@ cudaStream_t priority_stream() {
 // Run the QR of plan.X; the first run of a shape executes directly (so the
 // private arena grows to its final size) and then records the graph.
 void qr_run(Context& ctx, QrPlan& P) {
-    if (P.lookahead && P.capture) ctx.check_pending = true;
     if (P.exec) {
         NC_CUDA(cudaGraphLaunch(P.exec, ctx.stream));
         ctx.launches += P.kernels;

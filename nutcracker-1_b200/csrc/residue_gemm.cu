@@ -145,9 +145,6 @@ constexpr double kPh = high_part(kP), kPm = mid_part(kP), kPl = low_part(kP);
 constexpr int kBadExp = 1 << 30;         // exponent of a row with a non-finite element
 constexpr int kMaxK = 16000;             // |Re|, |Im| sums of K residue products fit in int32
 
-__device__ int g_res_error = 0;
-constexpr unsigned long long kWaitNs = 2000000000ull;
-
 // four values' low bytes
 __device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
@@ -464,6 +461,7 @@ struct ResGemm {
     int n4, mp;              // column groups of four and rows, padded to whole tiles
     uint32_t* res;           // [l][Re, Im][n4][mp] words of four columns
     ResidueGate gate;
+    const DeviceWatch* watch;
 };
 
 // v modulo p in [0, p] (p itself for some multiples of p), |v| < 2^31: the
@@ -517,6 +515,7 @@ residue_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
 
     if (warp == 0) {
         if (lane == 0) {
+            const bool mute = blockIdx.x == 0 && (P.watch->mute >> WATCH_RESIDUE & 1u);
             int t = 0;
             bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
@@ -524,10 +523,11 @@ residue_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
                 for (int c = 0; c < 3 && ok; ++c)
                     for (int kb = 0; kb < P.nkb; ++kb, ++t) {
                         const int s = t % STAGES;
-                        if (!mbar_wait(empty0 + 8 * s, ((uint32_t)(t / STAGES) & 1u) ^ 1u, kWaitNs, &g_res_error)) {
+                        if (!mbar_wait(empty0 + 8 * s, ((uint32_t)(t / STAGES) & 1u) ^ 1u, P.watch, WATCH_RESIDUE)) {
                             ok = false;
                             break;
                         }
+                        if (t == 0 && mute) continue;   // test switch: this stage never arrives
                         mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
                         tma_load_3d(base + s * STAGE_BYTES, &mapA, kb * TKB, m0, 3 * l + c, full0 + 8 * s);
                         tma_load_3d(base + s * STAGE_BYTES + A_STAGE, &mapB, kb * TKB, n0, 3 * l + c, full0 + 8 * s);
@@ -542,14 +542,14 @@ residue_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
                 for (int c = 0; c < 3 && ok; ++c, ++pass) {
                     const int b = pass & 1;
                     const uint32_t acc = tmem_d + (uint32_t)(b * TN);
-                    if (!mbar_wait(acce0 + 8 * b, ((uint32_t)(pass >> 1) & 1u) ^ 1u, kWaitNs, &g_res_error)) {
+                    if (!mbar_wait(acce0 + 8 * b, ((uint32_t)(pass >> 1) & 1u) ^ 1u, P.watch, WATCH_RESIDUE)) {
                         ok = false;
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     for (int kb = 0; kb < P.nkb; ++kb, ++t) {
                         const int s = t % STAGES;
-                        if (!mbar_wait(full0 + 8 * s, (uint32_t)(t / STAGES) & 1u, kWaitNs, &g_res_error)) {
+                        if (!mbar_wait(full0 + 8 * s, (uint32_t)(t / STAGES) & 1u, P.watch, WATCH_RESIDUE)) {
                             ok = false;
                             break;
                         }
@@ -578,7 +578,7 @@ residue_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
 #pragma unroll 1
             for (int c = 0; c < 3; ++c, ++pass) {
                 const int b = pass & 1;
-                ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (uint32_t)(pass >> 1) & 1u, kWaitNs, &g_res_error));
+                ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (uint32_t)(pass >> 1) & 1u, P.watch, WATCH_RESIDUE));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t src = tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * TN + h * EPI_COLS);
@@ -813,6 +813,7 @@ ResidueGate residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b
     G.mp = G.mt * TM;
     G.res = reinterpret_cast<uint32_t*>(ws + lay.res);
     G.gate = gate;
+    G.watch = ctx.watch;
     const CUtensorMap ma = make_map8(P.planes[0], lay.Kp, a.rows, a.rows, TM);
     const CUtensorMap mb = make_map8(P.planes[1], lay.Kp, b.rows, b.rows, TN);
     const long long items = (long long)G.mt * G.nt * NL;
@@ -828,7 +829,6 @@ ResidueGate residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b
     res_crt_kernel<<<dim3((G.M + 127) / 128, groups), 128, 0, ctx.stream>>>(G.res, o);
     NC_CHECK_LAUNCH();
     ctx.launches += 5;
-    ctx.check_pending = true;
     return gate;
 }
 
@@ -849,21 +849,6 @@ void zproduct(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResM
         q.gate = residue_product(ctx, a, b, lay, ws, p.C, I, sI, sn);
         zgemm_untimed(q, ctx);
     });
-}
-
-void device_check(Context& ctx) {
-    if (!ctx.check_pending) return;
-    ctx.check_pending = false;
-    NC_CUDA(cudaStreamSynchronize(ctx.stream));
-    int flag = 0;
-    NC_CUDA(cudaMemcpyFromSymbol(&flag, g_res_error, sizeof(int)));
-    if (flag) {
-        const int zero = 0;
-        NC_CUDA(cudaMemcpyToSymbol(g_res_error, &zero, sizeof(int)));
-    }
-    const int qr = qr_take_error();
-    if (flag) throw Error(NC_ERR_TIMEOUT, "residue GEMM: a pipeline wait exceeded its time limit");
-    if (qr) throw Error(NC_ERR_TIMEOUT, "cluster QR: an exchange between CTAs exceeded its time limit");
 }
 
 }  // namespace nc

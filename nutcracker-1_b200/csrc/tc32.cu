@@ -26,7 +26,7 @@
 // issues the TMA loads, warp 1 owns TMEM and issues the MMAs from one
 // thread.  The epilogue stores complex64 or complex128 to any strided
 // layout.  No multicast; every mbarrier wait is bounded by the global timer
-// and reports through g_tc_error.
+// and reports through the context's watch.
 #include <cstring>
 #include <string>
 
@@ -51,17 +51,11 @@ constexpr int TMEM_COLS = 512;       // two accumulator buffers of TN columns
 constexpr int CHUNK_KB = 2;          // K stages (per segment) per accumulator chunk
 constexpr size_t TC_SMEM = (size_t)STAGES * STAGE_BYTES + 1024 + 256;
 
-__device__ int g_tc_error = 0;
-// Limit of every mbarrier wait (2 s by default), and a test switch under
-// which tile (0,0,0) leaves its first K stage unloaded, so that its MMA
-// issuer's wait for that stage runs out and the failure path (g_tc_error,
-// NC_ERR_TIMEOUT on the host) can be exercised without a fault: every other
-// wait is bounded as well, no MMA has been issued, and the loads that were
-// issued complete long before the waits expire.  Both are set only by
-// tc_test_fault (nc_test_tc32_wait).
-__device__ unsigned long long g_tc_wait_ns = 2000000000ull;
-__device__ int g_tc_skip_first_load = 0;
-
+// Under the context's test switch (DeviceWatch::mute) tile (0,0,0) leaves its
+// first K stage unloaded, so that its MMA issuer's wait for that stage runs out
+// and the failure path (NC_ERR_TIMEOUT on the host) can be exercised without a
+// fault: every other wait is bounded as well, no MMA has been issued, and the
+// loads that were issued complete long before the waits expire.
 struct TcParams {
     int M, Nr, Kr, nkb;      // nkb: K stages per segment
     int nseg;                // 3 (3xTF32) or 1 (big x big)
@@ -69,6 +63,7 @@ struct TcParams {
     void* C;
     long long sm, sn, sz;
     int c_fp64;
+    const DeviceWatch* watch;
 };
 
 // kind::tf32 instruction descriptor: D f32, A/B tf32, both K-major, M x N.
@@ -98,7 +93,6 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN, z = blockIdx.z;
-    const unsigned long long limit = g_tc_wait_ns;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -128,7 +122,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
     if (warp == 0) {
         if (lane == 0) {
             const int zA = P.shareA ? 0 : z, zB = P.shareB ? 0 : z;
-            const bool skip_first = g_tc_skip_first_load && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
+            const bool skip_first = (P.watch->mute >> WATCH_TC32 & 1u) && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
             int t = 0;
             bool ok = true;
             for (int c = 0; c < nchunk && ok; ++c) {
@@ -137,7 +131,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
                     for (int kb = kb0; kb < kb1; ++kb, ++t) {
                         const int s = t % STAGES;
                         const uint32_t ph = (uint32_t)(t / STAGES) & 1u;
-                        if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, limit, &g_tc_error)) { ok = false; break; }
+                        if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, P.watch, WATCH_TC32)) { ok = false; break; }
                         if (skip_first && t == 0) continue;   // test switch: stage 0 never arrives
                         const CUtensorMap* ma = (seg == 2) ? &mapAs : &mapAb;
                         const CUtensorMap* mb = (seg == 1) ? &mapBs : &mapBb;
@@ -154,7 +148,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
             for (int c = 0; c < nchunk && ok; ++c) {
                 const int b = c & 1;
                 const uint32_t acc = tmem_d + (uint32_t)(b * TN);
-                if (!mbar_wait(acce0 + 8 * b, ((uint32_t)(c >> 1) & 1u) ^ 1u, limit, &g_tc_error)) break;   // buffer drained
+                if (!mbar_wait(acce0 + 8 * b, ((uint32_t)(c >> 1) & 1u) ^ 1u, P.watch, WATCH_TC32)) break;   // buffer drained
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const int kb0 = c * CHUNK_KB, kb1 = min(P.nkb, kb0 + CHUNK_KB);
                 bool first = true;
@@ -162,7 +156,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
                     for (int kb = kb0; kb < kb1; ++kb, ++t) {
                         const int s = t % STAGES;
                         const uint32_t ph = (uint32_t)(t / STAGES) & 1u;
-                        if (!mbar_wait(full0 + 8 * s, ph, limit, &g_tc_error)) { ok = false; break; }
+                        if (!mbar_wait(full0 + 8 * s, ph, P.watch, WATCH_TC32)) { ok = false; break; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint64_t da = smem_desc(base + s * STAGE_BYTES);
                         const uint64_t db = smem_desc(base + s * STAGE_BYTES + A_STAGE);
@@ -187,7 +181,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
         bool ok = true;
         for (int c = 0; c < nchunk; ++c) {
             const int b = c & 1;
-            ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (uint32_t)(c >> 1) & 1u, limit, &g_tc_error));   // warp-uniform
+            ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (uint32_t)(c >> 1) & 1u, P.watch, WATCH_TC32));   // warp-uniform
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -262,6 +256,7 @@ void tc_gemm(Context& ctx, const TcGemm& g) {
     P.nseg = g.three ? 3 : 1;
     P.shareA = shareA; P.shareB = shareB;
     P.C = g.C; P.sm = g.sm; P.sn = g.sn; P.sz = g.sz; P.c_fp64 = g.c_fp64 ? 1 : 0;
+    P.watch = ctx.watch;
     dim3 grid((g.M + TM - 1) / TM, (g.Nr + TN - 1) / TN, g.batch);
     NC_ARG(grid.y <= 65535 && grid.z <= 65535, "tc32: grid too large");
     const double flops = 2.0 * g.M * (double)g.Nr * g.Kr * P.nseg * g.batch;
@@ -270,23 +265,6 @@ void tc_gemm(Context& ctx, const TcGemm& g) {
         NC_CHECK_LAUNCH();
     });
     ctx.launches++;
-}
-
-void tc_test_fault(unsigned long long wait_ns, int skip_first_load) {
-    NC_ARG(wait_ns >= 1000, "tc32 wait limit must be at least 1 microsecond");
-    NC_CUDA(cudaMemcpyToSymbol(g_tc_wait_ns, &wait_ns, sizeof(wait_ns)));
-    NC_CUDA(cudaMemcpyToSymbol(g_tc_skip_first_load, &skip_first_load, sizeof(int)));
-}
-
-void tc_check(Context& ctx) {
-    NC_CUDA(cudaStreamSynchronize(ctx.stream));
-    int flag = 0;
-    NC_CUDA(cudaMemcpyFromSymbol(&flag, g_tc_error, sizeof(int)));
-    if (flag) {
-        const int zero = 0;
-        NC_CUDA(cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int)));
-        throw Error(NC_ERR_TIMEOUT, "tc32 GEMM: a pipeline wait exceeded its time limit");
-    }
 }
 
 }  // namespace nc

@@ -84,7 +84,32 @@ Context::Context() {
     NC_CUDA(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
     stream = own_stream;
     pinned_bytes = 1 << 16;
-    NC_CUDA(cudaMallocHost(&pinned, pinned_bytes));
+    NC_CUDA(cudaMallocHost(&pinned, pinned_bytes + sizeof(unsigned) * WATCH_KINDS));
+    expired = reinterpret_cast<volatile unsigned*>(static_cast<char*>(pinned) + pinned_bytes);
+    for (int k = 0; k < WATCH_KINDS; ++k) expired[k] = 0;
+    NC_CUDA(cudaMalloc(&watch, sizeof(DeviceWatch)));
+    set_watch(2000000000ull, 0);
+}
+
+void Context::set_watch(unsigned long long limit_ns, unsigned mute) {
+    NC_CUDA(cudaStreamSynchronize(stream));
+    const DeviceWatch w{limit_ns, mute, expired};
+    NC_CUDA(cudaMemcpyAsync(watch, &w, sizeof(w), cudaMemcpyHostToDevice, stream));
+    NC_CUDA(cudaStreamSynchronize(stream));
+}
+
+void Context::raise_expired() {
+    static const char* const what[WATCH_KINDS] = {"tc32 GEMM: a pipeline wait exceeded its time limit",
+                                                  "residue GEMM: a pipeline wait exceeded its time limit",
+                                                  "cluster QR: an exchange between CTAs exceeded its time limit"};
+    std::atomic_thread_fence(std::memory_order_acquire);
+    const char* message = nullptr;
+    for (int k = 0; k < WATCH_KINDS; ++k)
+        if (expired[k]) {
+            expired[k] = 0;
+            message = what[k];
+        }
+    if (message) throw Error(NC_ERR_TIMEOUT, message);
 }
 
 unsigned* Context::reduction_counter() {
@@ -112,6 +137,7 @@ Context::~Context() {
     if (ritz_ready) cudaEventDestroy(ritz_ready);
     if (ritz_done) cudaEventDestroy(ritz_done);
     if (red_counter) cudaFree(red_counter);
+    if (watch) cudaFree(watch);
     if (own_stream) cudaStreamDestroy(own_stream);
     if (pinned) cudaFreeHost(pinned);
 }
@@ -301,7 +327,7 @@ void znormalize_dev(Context& ctx, long long n, const cplx* nrm2sq_dev, cplx* x) 
 void read_scalars(Context& ctx, const void* dev, size_t bytes, void* host) {
     NC_ARG(bytes <= ctx.pinned_bytes, "read_scalars: too many bytes");
     NC_CUDA(cudaMemcpyAsync(ctx.pinned, dev, bytes, cudaMemcpyDeviceToHost, ctx.stream));
-    ctx.sync();
+    ctx.settle();
     memcpy(host, ctx.pinned, bytes);
 }
 
