@@ -116,9 +116,10 @@ int nc_tc_zgemm_dev(uint32_t M, uint32_t N, uint32_t K, const void* A_dev, const
    time limit of every bounded device wait of this thread's kernels (default
    2 s, here in nanoseconds, at least 1000): the tcgen05 GEMM's and the residue
    GEMM's pipelines and the exchange between the CTAs of a QR panel.  `mute` is
-   the sum of 1 (tcgen05 GEMM: tile (0,0,0) leaves its first K stage unloaded)
-   and 2 (residue GEMM: CTA 0 leaves its first K stage unloaded): a wait of
-   that kernel then runs out, it returns, and the next call of this thread
+   the sum of 1 (tcgen05 GEMM: tile (0,0,0) leaves its first K stage unloaded),
+   2 (residue GEMM: CTA 0 leaves its first K stage unloaded) and 4 (QR panel:
+   the last CTA does not send its sums of the first column): a wait of that
+   kernel then runs out, it returns, and the next call of this thread
    that waits for its work reports NC_ERR_TIMEOUT.  Restore (2000000000, 0)
    after use.  Waits for this thread's stream; returns a status code. */
 int nc_test_device_wait(uint64_t wait_ns, uint32_t mute);

@@ -653,7 +653,8 @@ cluster_subblock_qr_kernel(int mp, int nb, int rows_per_cta, cplx* __restrict__ 
     const int slice = (NB + C - 1) / C;   // columns per CTA of the exchanged V^H P
     const uint32_t bars = (uint32_t)__cvta_generic_to_shared(s.bar);
     const uint32_t column_bytes = (uint32_t)C * SB * 2 * 16 + SB * 16;   // sums of C CTAs, the pivot row
-    bool alive = true;
+    bool alive = true;   // this thread has not given up a wait
+    const bool mute = rank == C - 1 && (watch->mute >> WATCH_QR & 1u);   // test switch: no sums for column 0
     if (tid == 0) {
         for (int b = 0; b < 2; ++b) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * b) : "memory");
@@ -705,7 +706,7 @@ cluster_subblock_qr_kernel(int mp, int nb, int rows_per_cta, cplx* __restrict__ 
                 for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
                 // lane d (and d + 16) to CTA d
                 const int d = lane & 15;
-                if (d < C) {
+                if (d < C && !(mute && j == 0)) {
                     const uint32_t bar = remote(&s.bar[p], d);
                     send8(remote(&s.recv[p][c][2 * rank + h], d) + (up ? 8 : 0), sum, bar);
                     if (top && h == (j >> 5)) send8(remote(&s.piv[p][c], d) + (up ? 8 : 0), pv, bar);
@@ -761,8 +762,9 @@ cluster_subblock_qr_kernel(int mp, int nb, int rows_per_cta, cplx* __restrict__ 
                 s.G[jj][c] = cadd(pc, cmul(cconj(scale), Sc));   // v_jj^H v_c, column c holding v_c below its pivot
             }
             __syncthreads();
-            // every thread is past its wait: the barrier's next use is armed
-            if (tid == 0)
+            // every thread is past its wait: the barrier's next use is armed.  A thread that gave up does not
+            // arm it (its phase has not ended) but goes on: the cluster's barriers count every thread
+            if (tid == 0 && alive)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + 8 * p), "r"(column_bytes)
                              : "memory");
         }
@@ -863,6 +865,12 @@ cluster_subblock_qr_kernel(int mp, int nb, int rows_per_cta, cplx* __restrict__ 
     if (top)
         for (int q = tid; q < nb; q += CQ_T) tau_out[q] = s.taus[q];
     cluster.sync();   // no CTA leaves while another may still write its shared memory
+    if (!alive) {   // sums that nothing waited for may still be on their way: all are sent, 0.1 ms is ample
+        unsigned long long t0, t1;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+        do asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+        while (t1 - t0 < 100000ull);
+    }
 }
 
 // Cluster launch support (size CQ_MAXC needs the non-portable opt-in); a

@@ -486,8 +486,8 @@ residue_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     const uint32_t base = (raw + 1023u) & ~1023u;
     const uint32_t bars = base + STAGES * STAGE_BYTES;
     const uint32_t full0 = bars, empty0 = bars + 8 * STAGES;
-    const uint32_t accf0 = bars + 16 * STAGES, acce0 = accf0 + 16;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rg_smem_raw + (acce0 + 16 - raw));
+    const uint32_t accf0 = bars + 16 * STAGES, acce0 = accf0 + 16, drain = acce0 + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rg_smem_raw + (drain + 8 - raw));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -499,6 +499,7 @@ residue_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
             mbar_init(accf0 + 8 * b, 1);
             mbar_init(acce0 + 8 * b, EPI_WARPS);
         }
+        mbar_init(drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -533,6 +534,9 @@ residue_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
                         tma_load_3d(base + s * STAGE_BYTES + A_STAGE, &mapB, kb * TKB, n0, 3 * l + c, full0 + 8 * s);
                     }
             }
+            if (!ok)   // an expired wait: the loads in flight land before the shared memory is given back
+                for (int i = max(0, t - STAGES); i < t; ++i)
+                    mbar_wait(full0 + 8 * (i % STAGES), (uint32_t)(i / STAGES) & 1u, P.watch, WATCH_RESIDUE);
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -561,8 +565,12 @@ residue_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
                             mma_i8(acc, da + 2 * ks, db + 2 * ks, (kb | ks) ? 1u : 0u);
                         mma_commit(empty0 + 8 * s);
                     }
-                    mma_commit(accf0 + 8 * b);
+                    if (ok) mma_commit(accf0 + 8 * b);
                 }
+            if (!ok) {   // an expired wait: the MMAs issued end before the tensor memory is given back
+                mma_commit(drain);
+                mbar_wait(drain, 0, P.watch, WATCH_RESIDUE);
+            }
         }
     } else if (warp >= EPI_FIRST) {
         // epilogue: warp w drains TMEM lanes 32*(w%4) .. +31 (a warp can reach

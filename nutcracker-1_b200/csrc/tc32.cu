@@ -88,8 +88,8 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
     // full[S], empty[S], acc_full[2], acc_empty[2], TMEM slot
     const uint32_t bars = base + STAGES * STAGE_BYTES;
     const uint32_t full0 = bars, empty0 = bars + 8 * STAGES;
-    const uint32_t accf0 = bars + 16 * STAGES, acce0 = accf0 + 16;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tc_smem_raw + (acce0 + 16 - raw));
+    const uint32_t accf0 = bars + 16 * STAGES, acce0 = accf0 + 16, drain = acce0 + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tc_smem_raw + (drain + 8 - raw));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN, z = blockIdx.z;
@@ -103,6 +103,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
             mbar_init(accf0 + 8 * b, 1);
             mbar_init(acce0 + 8 * b, EPI_WARPS);
         }
+        mbar_init(drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -140,6 +141,9 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
                         tma_load_3d(base + s * STAGE_BYTES + A_STAGE, mb, kb * TK, n0, zB, full0 + 8 * s);
                     }
             }
+            if (!ok)   // an expired wait: the loads in flight land before the shared memory is given back
+                for (int i = max(0, t - STAGES); i < t; ++i)
+                    mbar_wait(full0 + 8 * (i % STAGES), (uint32_t)(i / STAGES) & 1u, P.watch, WATCH_TC32);
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -148,7 +152,7 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
             for (int c = 0; c < nchunk && ok; ++c) {
                 const int b = c & 1;
                 const uint32_t acc = tmem_d + (uint32_t)(b * TN);
-                if (!mbar_wait(acce0 + 8 * b, ((uint32_t)(c >> 1) & 1u) ^ 1u, P.watch, WATCH_TC32)) break;   // buffer drained
+                if (!mbar_wait(acce0 + 8 * b, ((uint32_t)(c >> 1) & 1u) ^ 1u, P.watch, WATCH_TC32)) { ok = false; break; }   // buffer drained
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const int kb0 = c * CHUNK_KB, kb1 = min(P.nkb, kb0 + CHUNK_KB);
                 bool first = true;
@@ -167,7 +171,11 @@ tc32_gemm_kernel(const __grid_constant__ CUtensorMap mapAb, const __grid_constan
                         }
                         mma_commit(empty0 + 8 * s);   // frees the stage once these MMAs have read it
                     }
-                mma_commit(accf0 + 8 * b);   // chunk complete in buffer b
+                if (ok) mma_commit(accf0 + 8 * b);   // chunk complete in buffer b
+            }
+            if (!ok) {   // an expired wait: the MMAs issued end before the tensor memory is given back
+                mma_commit(drain);
+                mbar_wait(drain, 0, P.watch, WATCH_TC32);
             }
         }
     } else {

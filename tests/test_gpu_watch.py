@@ -13,6 +13,7 @@ from gpu_util import device_rand, heff_dev
 pytestmark = pytest.mark.gpu
 TIMEOUT = 1004
 RESIDUE = 2
+QR = 4
 
 
 @pytest.fixture()
@@ -78,3 +79,50 @@ def test_residue_gemm_recovers(lib):
     assert lib.lib.nc_synchronize() == TIMEOUT
     assert lib.lib.nc_test_device_wait(ct.c_uint64(2_000_000_000), ct.c_uint32(0)) == 0
     assert torch.equal(heff_dev(lib, *args), ref)
+
+
+@pytest.mark.parametrize("bl,bm", [(60, 96), (130, 125), (520, 515)])
+def test_qr_panel_recovers(lib, bl, bm):
+    """One to nine CTAs a panel; the first call runs the panels directly, the
+    second from the recorded graph, with the waits running out in both."""
+    import torch
+    from gpu_util import device_pointers
+
+    A, B = device_rand((2, bl, bm), 1), device_rand((2, bm, 70), 2)
+    dims = [ct.c_uint32(v) for v in (bl, bm, 70, 2, 2)]
+
+    def move():
+        oA, oB = torch.empty_like(A), torch.empty_like(B)
+        torch.cuda.synchronize()
+        status = lib.lib.nc_gauge_move_dev(ct.c_int(1), *dims, *device_pointers(A, B, oA, oB))
+        return status, oA, oB
+
+    for _ in range(2):
+        _mute(lib, QR)
+        assert move()[0] == 0
+        assert lib.lib.nc_synchronize() == TIMEOUT and b"cluster QR" in lib.lib.nc_last_error()
+        assert lib.lib.nc_synchronize() == 0
+    assert lib.lib.nc_test_device_wait(ct.c_uint64(2_000_000_000), ct.c_uint32(0)) == 0
+    status, oA, oB = move()
+    assert status == 0 and lib.lib.nc_synchronize() == 0
+    eye = torch.eye(bm, dtype=A.dtype, device="cuda")
+    assert float((torch.einsum("alm,aln->mn", oA, oA.conj()) - eye).norm() / eye.norm()) < 1e-12
+    ref = torch.einsum("alm,bmr->albr", A, B)
+    assert float((torch.einsum("alm,bmr->albr", oA, oB) - ref).norm() / ref.norm()) < 1e-12
+
+
+def test_host_buffer_call_reports(lib):
+    """A call on host buffers waits for its own work: it reports, and the next one is right."""
+    import numpy as np
+
+    rng = np.random.default_rng(3)
+    A = np.asfortranarray(rng.normal(size=(100, 90, 2)) + 1j * rng.normal(size=(100, 90, 2)))   # (bm, bl, d)
+    B = np.asfortranarray(rng.normal(size=(60, 100, 2)) + 1j * rng.normal(size=(60, 100, 2)))
+    args = (90, 100, 60, 2, 2, A, B)
+    good = lib.Core.norm_denorm_going_right(*args)
+    _mute(lib, QR)
+    with pytest.raises(lib.NutcrackerError, match="cluster QR"):
+        lib.Core.norm_denorm_going_right(*args)
+    assert lib.lib.nc_test_device_wait(ct.c_uint64(2_000_000_000), ct.c_uint32(0)) == 0
+    again = lib.Core.norm_denorm_going_right(*args)
+    assert all(np.array_equal(x, y) for x, y in zip(good[-2:], again[-2:]))
