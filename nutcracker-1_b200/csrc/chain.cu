@@ -661,6 +661,7 @@ struct Chain {
             cur_site[i - 1] = std::move(a);
             cur_site[i] = std::move(b);
         }
+        ctx.settle();   // a growth that went wrong leaves the chain as it was
         bonds = nb;
         bandwidth = new_b;
         // re-allocate environments for the new bonds and rebuild them from the right
@@ -675,7 +676,7 @@ struct Chain {
         for (int i = N - 1; i >= 1; --i) absorb_right(i);
         cur = 0;
         reset_projector_matrix();
-        NC_CUDA(cudaStreamSynchronize(ctx.stream));
+        ctx.settle();
     }
 
     void optimize_chain() {
@@ -721,7 +722,7 @@ struct Chain {
         }
         if (!proj[0].right.p) proj[0].right.alloc(1);
         if (!proj[N - 1].left.p) proj[N - 1].left.alloc(1);
-        NC_CUDA(cudaStreamSynchronize(ctx.stream));
+        ctx.settle();
         projectors.push_back(std::move(proj));
     }
 
@@ -1004,7 +1005,7 @@ int nc_chain_get_site(nc_chain* c, uint32_t i, nc_complex* out, uint32_t* dims) 
         if (out) {
             NC_CUDA(cudaMemcpyAsync(out, ch.site[i].p, ch.site_elems(i) * sizeof(cplx), cudaMemcpyDeviceToHost,
                                     ch.ctx.stream));
-            NC_CUDA(cudaStreamSynchronize(ch.ctx.stream));
+            ch.ctx.settle();
         }
     })
 }

@@ -398,7 +398,7 @@ int convert_vectors_to_reflectors_dev(Context& ctx, long long m, int n, cplx* A,
     for (int c = 0; c < n; ++c)
         NC_CUDA(cudaMemcpyAsync(R.data() + (size_t)c * k, A + (size_t)c * m, k * sizeof(cplx),
                                 cudaMemcpyDeviceToHost, ctx.stream));
-    NC_CUDA(cudaStreamSynchronize(ctx.stream));
+    ctx.settle();
     std::vector<double> norms(k);
     for (int i = 0; i < k; ++i) {
         double a = 0;

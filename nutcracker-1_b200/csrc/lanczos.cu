@@ -520,6 +520,7 @@ class RitzLane {
             std::atomic_thread_fence(std::memory_order_acquire);
         }
         on_ = nullptr;
+        ctx_.raise_expired();   // a product behind this result gave up a wait
         return *out_;
     }
 

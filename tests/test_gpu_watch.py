@@ -126,3 +126,33 @@ def test_host_buffer_call_reports(lib):
     assert lib.lib.nc_test_device_wait(ct.c_uint64(2_000_000_000), ct.c_uint32(0)) == 0
     again = lib.Core.norm_denorm_going_right(*args)
     assert all(np.array_equal(x, y) for x, y in zip(good[-2:], again[-2:]))
+
+
+def test_chain_calls_report(lib):
+    """A chain's calls that hand out or keep the state answer for the moves that
+    made it; a growth that went wrong leaves the chain as it was."""
+    import numpy as np
+    from nutcracker_b200 import operators
+    from nutcracker_b200.chain import Chain
+
+    chain = Chain(operators.heisenberg(14), initial_bandwidth_dimension=80, seed=3)
+    chain.perform_optimization_sweep()
+    energy = chain.get_energy()
+    site = chain.get_site(0)
+    _mute(lib, QR)
+    with pytest.raises(lib.NutcrackerError, match="cluster QR"):
+        chain.increase_bandwidth_dimension(100)
+    with pytest.raises(lib.NutcrackerError, match="cluster QR"):
+        chain.construct_and_add_projector_from_state()
+    assert lib.lib.nc_test_device_wait(ct.c_uint64(2_000_000_000), ct.c_uint32(0)) == 0
+    info = chain.info()
+    assert info["bandwidth_dimension"] == 80 and info["number_of_projectors"] == 0
+    assert np.array_equal(chain.get_site(0), site)
+    assert abs(chain.compute_expectation_value() - energy) < 1e-9 * abs(energy)
+    chain.increase_bandwidth_dimension(100)
+    assert abs(chain.compute_expectation_value() - energy) < 1e-9 * abs(energy)
+    _mute(lib, QR)
+    chain.move_to(7)
+    assert lib.lib.nc_test_device_wait(ct.c_uint64(2_000_000_000), ct.c_uint32(0)) == 0
+    with pytest.raises(lib.NutcrackerError, match="cluster QR"):
+        chain.get_site(7)
