@@ -69,6 +69,9 @@ class Arena {
     void* alloc(size_t bytes);
     template <class T>
     T* alloc_n(size_t n) { return static_cast<T*>(alloc(n * sizeof(T))); }
+    // Whether `bytes` can be had, in one piece or as parts of it allocated next;
+    // nothing is taken.
+    bool reserve(size_t bytes);
     struct Mark { size_t block, used; };
     Mark mark() const;
     void release(Mark m);

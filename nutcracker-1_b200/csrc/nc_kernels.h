@@ -66,8 +66,9 @@ ZGemmParams zgemm_params(int opA, int opB, int M, int N, int K, const cplx* A, l
 void zgemm(const ZGemmParams& p, cudaStream_t s);
 // Launch with automatic split-K when the tile grid is small (workspace from ctx.arena).
 void zgemm(const ZGemmParams& p, Context& ctx);
-// The same without an entry in nc_profile_*.
+// The same without an entry in nc_profile_*; its workspace.
 void zgemm_untimed(const ZGemmParams& p, Context& ctx);
+size_t zgemm_workspace_bytes(const ZGemmParams& p);
 void scale_strided(const ZGemmParams& p, cudaStream_t s);
 
 // One MPO site on the device: W (d,d,nnz) column-major, idx (2,nnz) 1-based.
@@ -200,7 +201,8 @@ bool residue_gemm_pays(long long M, long long N, long long K);
 double residue_scratch_bytes(long long M, long long N, long long K);
 // zgemm(p) (alpha 1, beta 0), written a second time as C(m,n) = sum_k A(m,k)
 // B(n,k) to p.C[(m % I) + (m / I) * sI + n * sn]: through residues where that
-// pays and holds the operands (scratch from ctx.scratch()).
+// pays and holds the operands (scratch from ctx.scratch(); where that cannot be
+// had the product is zgemm(p)).
 void zproduct(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResMatrix& b, int I, long long sI,
               long long sn);
 

@@ -851,6 +851,10 @@ void zproduct(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResM
         return;
     }
     const ResLayout lay(a, b);
+    if (!ctx.scratch().reserve(lay.bytes + zgemm_workspace_bytes(p) + 256)) {
+        zgemm(p, ctx);   // the memory is taken: the product that needs (almost) none
+        return;
+    }
     profile_launch(ctx, 8.0 * a.rows * (double)b.rows * a.K, 0, [&] {
         ZGemmParams q = p;
         char* ws = ctx.scratch().alloc_n<char>(lay.bytes);

@@ -57,6 +57,18 @@ void* Arena::alloc(size_t bytes) {
     return b.p;
 }
 
+bool Arena::reserve(size_t bytes) {
+    const Mark m = mark();
+    try {
+        alloc(bytes);
+    } catch (const Error& e) {
+        if (e.code != NC_ERR_NOMEM) throw;
+        return false;
+    }
+    release(m);
+    return true;
+}
+
 Arena::Mark Arena::mark() const {
     if (blocks_.empty()) return Mark{0, 0};
     return Mark{blocks_.size(), blocks_.back().used};

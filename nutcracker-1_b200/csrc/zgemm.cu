@@ -258,11 +258,10 @@ void zgemm(const ZGemmParams& p, Context& ctx) {
     profile_launch(ctx, flops, 0, [&] { zgemm_untimed(p, ctx); });
 }
 
-void zgemm_untimed(const ZGemmParams& p_in, Context& ctx) {
-    ZGemmParams p = p_in;
-    if (p.M <= 0 || p.N <= 0 || p.batch <= 0) return;
-    if (p.nb0 <= 0) p.nb0 = p.batch;
-    // Split K when the tile grid cannot fill the 148 SMs and K is long.
+namespace {
+// Split K when the tile grid cannot fill the 148 SMs and K is long, or where
+// the caller wants short chains.
+int split_k(const ZGemmParams& p, int& kchunk) {
     const long long tiles = (long long)ceil_div(p.M, 64) * ceil_div(p.N, 64) * p.batch;
     int nsplit = 1;
     if (p.K >= 256 && tiles < 2 * 148) {
@@ -270,13 +269,30 @@ void zgemm_untimed(const ZGemmParams& p_in, Context& ctx) {
         nsplit = std::max(1, std::min(nsplit, 32));
     }
     if (p.chain > 0) nsplit = std::max(nsplit, (p.K + p.chain - 1) / p.chain);
+    if (nsplit <= 1) return 1;
+    kchunk = (int)(((p.K + nsplit - 1) / nsplit + 15) / 16 * 16);
+    return (p.K + kchunk - 1) / kchunk;
+}
+}  // namespace
+
+size_t zgemm_workspace_bytes(const ZGemmParams& p) {
+    if (p.M <= 0 || p.N <= 0 || p.batch <= 0) return 0;
+    int kchunk = 0;
+    const int nsplit = split_k(p, kchunk);
+    return nsplit > 1 ? sizeof(cplx) * (size_t)p.M * p.N * p.batch * nsplit : 0;
+}
+
+void zgemm_untimed(const ZGemmParams& p_in, Context& ctx) {
+    ZGemmParams p = p_in;
+    if (p.M <= 0 || p.N <= 0 || p.batch <= 0) return;
+    if (p.nb0 <= 0) p.nb0 = p.batch;
+    int kchunk = 0;
+    const int nsplit = split_k(p, kchunk);
     if (nsplit <= 1) {
         zgemm(p, ctx.stream);
         ctx.launches++;
         return;
     }
-    int kchunk = (int)(((p.K + nsplit - 1) / nsplit + 15) / 16 * 16);
-    nsplit = (p.K + kchunk - 1) / kchunk;
     ArenaFrame f(ctx.scratch());
     const long long mn = (long long)p.M * p.N;
     cplx* ws = ctx.scratch().alloc_n<cplx>((size_t)mn * p.batch * nsplit);
