@@ -13,7 +13,9 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <set>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "nc_abi_util.h"
@@ -755,7 +757,9 @@ struct Chain {
     // `bandwidth` for `levels` levels: the buffers allocate_for_bonds and the
     // projector sites hold, plus the solver's arena peak (Lanczos basis,
     // H_eff scratch, the residue products' or the precision form's tensor-core
-    // operands) and the gauge moves' QR plans, with a 25% margin.
+    // operands) and the gauge moves' QRs (one plan a shape and direction), with
+    // a 25% margin.  The arena counts twice: its blocks are shared by requests of
+    // many sizes (22 sites at 512: 2.35 GB taken, 2.8 GB estimated).
     static uint64_t footprint_bytes(const std::vector<int>& d, const std::vector<int>& cl, const std::vector<int>& cr,
                                     int bandwidth, int levels, int krylov, int precision) {
         const int n = (int)d.size();
@@ -776,20 +780,27 @@ struct Chain {
                                        residue_scratch_bytes(bl * cl[i], bl, br * d[i])})
                 residue = std::max(residue, bytes);
         }
-        elems += residue / sizeof(cplx);
+        double arena = residue / sizeof(cplx);
         elems += (n + 2) * maxs;                                   // sites and spares
         const int np = std::max(0, levels - 1);
         for (int i = 0; i < n; ++i)                                // projector sites and overlap environments
             elems += np * (3.0 * bonds[i] * bonds[i + 1] * d[i] + (double)bonds[i] * bonds[i] +
                            (double)bonds[i + 1] * bonds[i + 1]);
-        elems += (krylov + 1 + std::max(4, krylov / 3) + 4) * maxs;   // Lanczos basis, restart vectors
-        elems += 2.0 * maxs * 8 + maxenv;                         // H_eff / environment-update scratch
-        double qr = 0;
-        for (int i = 0; i + 1 < n; ++i) {                          // largest gauge QR plan (m x n, Q accumulated m x m)
-            const double m = (double)bonds[i] * d[i], k = bonds[i + 1];
-            qr = std::max(qr, 4.0 * m * k + m * m + 2.0 * k * k);
+        arena += (krylov + 1 + std::max(4, krylov / 3) + 4) * maxs;   // Lanczos basis, restart vectors
+        arena += 2.0 * maxs * 8 + maxenv;                         // H_eff / environment-update scratch
+        std::set<std::pair<int, int>> plans[2];                    // gauge QR plans, moving right and left
+        double plan = 0, scratch = 0;
+        for (int i = 0; i + 1 < n; ++i) {
+            plans[0].insert({bonds[i] * d[i], bonds[i + 1]});
+            plans[1].insert({bonds[i + 2] * d[i + 1], bonds[i + 1]});
         }
-        elems += 2 * qr;
+        for (const auto& direction : plans)
+            for (const auto& mk : direction) {
+                plan += qr_plan_bytes(mk.first, mk.second);
+                scratch = std::max(scratch, qr_scratch_bytes(mk.first, mk.second));
+            }
+        arena += scratch / sizeof(cplx);
+        elems += plan / sizeof(cplx) + 2 * arena;
         if (precision) elems += 3.0 * maxenv + 4.0 * maxs;       // TF32 pairs of environments and sites (float = elems/4)
         return (uint64_t)(1.25 * elems * sizeof(cplx)) + (64ull << 20);
     }

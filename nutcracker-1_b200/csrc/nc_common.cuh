@@ -64,6 +64,13 @@ __host__ __device__ inline double cabs2(cplx a) { return a.x * a.x + a.y * a.y; 
 class Arena {
    public:
     Arena() {}
+    // Blocks of exactly what is asked for, for an owner that asks once.
+    static Arena exact() {
+        Arena a;
+        a.exact_ = true;
+        return a;
+    }
+    Arena(Arena&&) = default;
     ~Arena();
     // Bump-allocate `bytes` (256-byte aligned) from the current frame.
     void* alloc(size_t bytes);
@@ -81,6 +88,7 @@ class Arena {
     struct Block { char* p; size_t size; size_t used; };
     std::vector<Block> blocks_;   // live blocks, last one is the bump target
     std::vector<Block> spare_;    // released blocks kept for reuse (never freed while live)
+    bool exact_ = false;
 };
 
 // RAII frame over an Arena.

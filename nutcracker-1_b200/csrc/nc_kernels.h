@@ -162,6 +162,10 @@ int convert_vectors_to_reflectors_dev(Context& ctx, long long m, int n, cplx* A,
 // triangle of A; optional explicit Q (m x n) and R (n x n, zeros below,
 // conjugated if conjR).
 void householder_qr(Context& ctx, int m, int n, cplx* A, cplx* Q, cplx* R, bool conjR);
+// Device bytes of a gauge move's m x n QR: what each shape keeps for the life
+// of the thread, and what all shapes share.
+double qr_plan_bytes(int m, int n);
+double qr_scratch_bytes(int m, int n);
 
 // ---- tcgen05 3xTF32 complex GEMM (tc32.cu) ---------------------------------
 // One operand of the real GEMM: rows x Kr floats, Kr contiguous, row stride

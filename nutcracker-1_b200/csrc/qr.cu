@@ -1093,22 +1093,20 @@ void householder_qr(Context& ctx, int m, int n, cplx* A, cplx* Q, cplx* R, bool 
 // 1.36e-14 / 9.2e-15, |A - QR| / |A| 8.2e-16 / 1.04e-15 / 7.4e-16,
 // |R^H R - A^H A| / |A|^2 5.8e-17 / 9.5e-17 / 6.5e-17.
 constexpr int kDotChain = 32;
-void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int m, int n, cplx* A, cplx* Q,
+// V (m x n, the reflectors) and T (n x n) are what qr_form_q takes.
+void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int m, int n, cplx* A, cplx* V, cplx* T,
                               cplx* R, bool conjR) {
     NC_ARG(m >= n && n >= 1 && m <= CQ_MAXC * CQ_MAXR, "householder_qr: need 1 <= n <= m <= 2048");
     Arena& ar = ctx.scratch();
     ArenaFrame f(ar);
     const long long lda = m;
     const int nblocks = (n + NB - 1) / NB;
-    cplx* V = ar.alloc_n<cplx>((size_t)m * n);
     cplx* tau = ar.alloc_n<cplx>(n);
     cplx* GW = ar.alloc_n<cplx>((size_t)nblocks * 2 * NB * NB);   // per block: V^H V, V^H A_{k+1}
     cplx* W2m = ar.alloc_n<cplx>(NB * NB);
     cplx* Tb = ar.alloc_n<cplx>(NB * NB);
     cplx* Ws = ar.alloc_n<cplx>((size_t)NB * n);
     cplx* W2s = ar.alloc_n<cplx>((size_t)NB * n);
-    cplx* T = ar.alloc_n<cplx>((size_t)n * n);
-    cplx* Z = ar.alloc_n<cplx>((size_t)n * n);
     const uint64_t side0 = side.launches;
     NC_SET_SMEM_ONCE(reflector_solve_kernel, TRS_SMEM);
 
@@ -1169,7 +1167,6 @@ void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int 
             zgemm(p, side);
         }
         NC_CUDA(cudaEventRecord(ev_bulk, side.stream));
-        if (!Q) continue;
         place_t_kernel<<<1, 256, 0, side.stream>>>(nb, Tb, T + j0 + j0 * (long long)n, n);
         NC_CHECK_LAUNCH();
         side.launches++;
@@ -1192,8 +1189,12 @@ void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int 
         NC_CHECK_LAUNCH();
         ctx.launches++;
     }
-    if (!Q) return;
-    // Z = T V_1^H, Q = I - V Z
+}
+
+// Q (m x n) = I - V (T V_1^H).
+void qr_form_q(Context& ctx, int m, int n, const cplx* V, const cplx* T, cplx* Q) {
+    ArenaFrame f(ctx.scratch());
+    cplx* Z = ctx.scratch().alloc_n<cplx>((size_t)n * n);
     ResMatrix a, b;
     a.X = T; a.rows = n; a.K = n; a.si = 1; a.sk = n; a.I = n;
     b.X = V; b.rows = n; b.K = n; b.si = 1; b.sk = m; b.I = n; b.conj = 1;
@@ -1206,6 +1207,22 @@ void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int 
     ctx.launches++;
 }
 
+double qr_plan_bytes(int m, int n) {
+    const double k = n, chunks = (m + kDotChain - 1) / kDotChain;
+    double q = 0;   // Q's products where they are part of the graph: T V_1^H and split-K partials
+    if (residue_scratch_bytes(n, n, n) + residue_scratch_bytes(m, n, n) == 0)
+        q = sizeof(cplx) * k * k +
+            (double)std::max(zgemm_workspace_bytes(zgemm_params(OP_N, OP_C, n, n, n, nullptr, n, nullptr, m, nullptr, n)),
+                             zgemm_workspace_bytes(zgemm_params(OP_N, OP_N, m, n, n, nullptr, m, nullptr, n, nullptr, m)));
+    const double panel = 2.0 * NB * NB * ((n + NB - 1) / NB) + 2.0 * NB * NB * (chunks + 1);   // per block; partials and one T
+    return sizeof(cplx) * (3.0 * m * k + 2.0 * k * k + (2.0 * NB + 1) * k + panel) + q + 16384.0;
+}
+
+double qr_scratch_bytes(int m, int n) {
+    const double k = n, chunks = (m + kDotChain - 1) / kDotChain;
+    return sizeof(cplx) * (k * k + NB * k * chunks) + std::max(residue_scratch_bytes(n, n, n), residue_scratch_bytes(m, n, n));
+}
+
 // ---------------------------------------------------------------------------
 // gauge moves (core.f95:2708-2960 semantics, QR gauge)
 // ---------------------------------------------------------------------------
@@ -1214,22 +1231,25 @@ void householder_qr_lookahead(Context& ctx, Context& side, cudaEvent_t* ev, int 
 // hundred short kernels (the panels are latency bound), so replaying a
 // pre-recorded graph removes the per-launch host overhead.  The plan owns its
 // input/output buffers and a private workspace arena, so the pointers baked
-// into the graph stay valid and are never shared with other work.
+// into the graph stay valid and are never shared with other work.  Q's products
+// are part of the graph unless their integers need scratch of several times the
+// matrix: then they follow it, with the context's scratch, which every shape shares.
 struct QrPlan {
     const Context* owner = nullptr;   // its graph reports expired waits to this context
     int m = 0, n = 0;
     bool conjR = false;
-    Arena arena;
-    // look-ahead: the thread's second stream (side_context) with this plan's
-    // split-K arena, and the plan's events
+    Arena arena = Arena::exact();
+    // look-ahead: the thread's second stream (side_context, whose arena every
+    // plan's graph uses) and the plan's events
     bool lookahead = false;
-    Arena side_arena;
     std::vector<cudaEvent_t> ev;
     // single-block shapes are run directly: recording a graph saves nothing
     bool capture = true;
     cplx* X = nullptr;   // input (m x n), overwritten
     cplx* Q = nullptr;   // explicit Q (m x n)
     cplx* R = nullptr;   // R (n x n), conjugated if conjR
+    cplx* V = nullptr;   // reflectors (m x n) and compact-WY factor (n x n), look-ahead form only
+    cplx* T = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint64_t kernels = 0;
@@ -1255,6 +1275,7 @@ QrPlan& qr_plan(Context& ctx, int m, int n, bool conjR) {
     auto p = std::make_unique<QrPlan>();
     p->owner = &ctx;
     p->m = m; p->n = n; p->conjR = conjR;
+    p->arena.reserve((size_t)qr_plan_bytes(m, n));
     p->X = p->arena.alloc_n<cplx>((size_t)m * n);
     p->Q = p->arena.alloc_n<cplx>((size_t)m * n);
     p->R = p->arena.alloc_n<cplx>((size_t)n * n);
@@ -1264,6 +1285,10 @@ QrPlan& qr_plan(Context& ctx, int m, int n, bool conjR) {
         for (cudaEvent_t& e : p->ev) NC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     p->capture = n > NB;
+    if (p->lookahead && p->capture) {
+        p->V = p->arena.alloc_n<cplx>((size_t)m * n);
+        p->T = p->arena.alloc_n<cplx>((size_t)n * n);
+    }
     plans.push_back(std::move(p));
     return *plans.back();
 }
@@ -1288,23 +1313,26 @@ cudaStream_t priority_stream() {
     return s;
 }
 
+bool q_after(const QrPlan& P) { return residue_gemm_pays(P.n, P.n, P.n) || residue_gemm_pays(P.m, P.n, P.n); }
+
 // Run the QR of plan.X; the first run of a shape executes directly (so the
 // private arena grows to its final size) and then records the graph.
 void qr_run(Context& ctx, QrPlan& P) {
     if (P.exec) {
         NC_CUDA(cudaGraphLaunch(P.exec, ctx.stream));
         ctx.launches += P.kernels;
+        if (P.lookahead && q_after(P)) qr_form_q(ctx, P.m, P.n, P.V, P.T, P.Q);
         return;
     }
     const bool prof = ctx.profile;
     ctx.profile = false;
     ctx.ws_override = &P.arena;
     Context& side = side_context();
-    side.ws_override = &P.side_arena;
     auto once = [&] {
-        if (P.lookahead && P.capture)
-            householder_qr_lookahead(ctx, side, P.ev.data(), P.m, P.n, P.X, P.Q, P.R, P.conjR);
-        else
+        if (P.lookahead && P.capture) {
+            householder_qr_lookahead(ctx, side, P.ev.data(), P.m, P.n, P.X, P.V, P.T, P.R, P.conjR);
+            if (!q_after(P)) qr_form_q(ctx, P.m, P.n, P.V, P.T, P.Q);
+        } else
             householder_qr(ctx, P.m, P.n, P.X, P.Q, P.R, P.conjR);
     };
     if (!P.capture) {
@@ -1355,6 +1383,7 @@ void qr_run(Context& ctx, QrPlan& P) {
     }
     ctx.ws_override = nullptr;
     ctx.profile = prof;
+    if (P.lookahead && q_after(P)) qr_form_q(ctx, P.m, P.n, P.V, P.T, P.Q);
 }
 }  // namespace
 

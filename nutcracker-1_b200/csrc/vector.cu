@@ -27,18 +27,24 @@ void* Arena::alloc(size_t bytes) {
             return p;
         }
     }
-    // reuse a spare block large enough, else allocate a new one
-    for (size_t i = 0; i < spare_.size(); ++i) {
-        if (spare_[i].size >= bytes) {
-            Block b = spare_[i];
-            spare_.erase(spare_.begin() + i);
-            b.used = bytes;
-            blocks_.push_back(b);
-            return b.p;
-        }
+    // reuse the smallest spare block that is large enough (a small request must
+    // not take the block that a large one will need), else allocate a new one
+    size_t fit = spare_.size();
+    for (size_t i = 0; i < spare_.size(); ++i)
+        if (spare_[i].size >= bytes && (fit == spare_.size() || spare_[i].size < spare_[fit].size)) fit = i;
+    if (fit < spare_.size()) {
+        Block b = spare_[fit];
+        spare_.erase(spare_.begin() + fit);
+        b.used = bytes;
+        blocks_.push_back(b);
+        return b.p;
     }
     size_t last = blocks_.empty() ? 0 : blocks_.back().size;
-    size_t sz = std::max(bytes, std::max(last * 2, size_t(64) << 20));
+    // small requests share blocks that double up to 256 MB; a large one gets a block of its own, with a quarter to grow into
+    const size_t shared = size_t(256) << 20;
+    size_t sz = exact_ ? bytes
+                       : std::max(bytes > shared / 2 ? bytes + bytes / 4 : bytes,
+                                  std::max(std::min(last * 2, shared), size_t(64) << 20));
     Block b;
     cudaError_t e = cudaMalloc(&b.p, sz);
     if (e != cudaSuccess) {
