@@ -794,12 +794,17 @@ struct Chain {
             plans[0].insert({bonds[i] * d[i], bonds[i + 1]});
             plans[1].insert({bonds[i + 2] * d[i + 1], bonds[i + 1]});
         }
+        double absorb = 0;                                         // the neighbour's product with the factor
+        for (int i = 0; i + 1 < n; ++i) {
+            absorb = std::max(absorb, residue_scratch_bytes(bonds[i + 2] * d[i + 1], bonds[i + 1], bonds[i + 1]));
+            absorb = std::max(absorb, residue_scratch_bytes(bonds[i + 1], bonds[i] * d[i], bonds[i + 1]));
+        }
         for (const auto& direction : plans)
             for (const auto& mk : direction) {
                 plan += qr_plan_bytes(mk.first, mk.second);
                 scratch = std::max(scratch, qr_scratch_bytes(mk.first, mk.second));
             }
-        arena += scratch / sizeof(cplx);
+        arena += (scratch + absorb) / sizeof(cplx);
         elems += plan / sizeof(cplx) + 2 * arena;
         if (precision) elems += 3.0 * maxenv + 4.0 * maxs;       // TF32 pairs of environments and sites (float = elems/4)
         return (uint64_t)(1.25 * elems * sizeof(cplx)) + (64ull << 20);

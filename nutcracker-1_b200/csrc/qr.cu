@@ -1388,25 +1388,34 @@ void qr_run(Context& ctx, QrPlan& P) {
 }  // namespace
 
 // The absorption GEMM of the gauge factor, on ctx.stream or, with `as`, on
-// the second stream after the QR that produced the factor.  A product that pays
-// through residues (a, b: the same one) runs on ctx.stream in either case: it
-// needs the context's scratch, and it is shorter than what it would hide behind
-// (chi = 1024: 605 us on the FP64 pipe, 160 through residues, B200).
+// the second stream after the QR that produced the factor: there it takes the
+// second context's scratch (no QR runs beside it) and reports to ctx.
 static void absorb_factor(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResMatrix& b, int I,
                           long long sI, long long sn, const AbsorbAsync* as) {
-    if (residue_gemm_pays(a.rows, b.rows, a.K)) {
-        zproduct(ctx, p, a, b, I, sI, sn);
-        if (as) NC_CUDA(cudaEventRecord(as->done, ctx.stream));
-        return;
-    }
     if (!as) {
-        zgemm(p, ctx);
+        zproduct(ctx, p, a, b, I, sI, sn);
         return;
     }
     NC_CUDA(cudaEventRecord(as->ready, ctx.stream));
     NC_CUDA(cudaStreamWaitEvent(as->stream, as->ready, 0));
-    zgemm(p, as->stream);
-    ctx.launches++;
+    if (residue_gemm_pays(a.rows, b.rows, a.K)) {
+        struct OnStream {   // the second context's work on another stream, for the life of this object
+            Context& c;
+            cudaStream_t s;
+            DeviceWatch* w;
+            OnStream(Context& side, const Context& ctx, cudaStream_t on) : c(side), s(side.stream), w(side.watch) {
+                c.stream = on;
+                c.watch = ctx.watch;
+            }
+            ~OnStream() { c.stream = s; c.watch = w; }
+        } on(side_context(), ctx, as->stream);
+        const uint64_t l0 = on.c.launches;
+        zproduct(on.c, p, a, b, I, sI, sn);
+        ctx.launches += on.c.launches - l0;
+    } else {
+        zgemm(p, as->stream);
+        ctx.launches++;
+    }
     NC_CUDA(cudaEventRecord(as->done, as->stream));
 }
 
