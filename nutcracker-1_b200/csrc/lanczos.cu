@@ -663,17 +663,22 @@ int optimize_site(Context& ctx, int bl, int br, const MpoSite& op, const cplx* L
         NC_CHECK_LAUNCH();
         ctx.launches++;
     };
-    // The projected problem is one block of latency (65 us at 14 to 24 vectors
-    // on a B200), as long as a small site's whole product and
+    // The projected problem is one block of latency (47 us in the mean of a
+    // 24-vector solve on a B200), as long as a small site's whole product and
     // orthogonalisation, and the next step needs nothing of it but whether to
     // go on.  So on sites of at most 2^17 elements, from six vectors up and
     // while the last residual is still 30 times the tolerance, it runs on a
     // stream of its own and the next step starts beside it; a step that turns
     // out not to be needed is dropped (the result only reads V_0 .. V_j).  The
-    // residual rule keeps that rare: a step seldom gains a factor of 30.  Site
-    // solve 48 x 48 x 2: 5.6 -> 3.9 ms; a 20-site sweep, chi <= 64, whose steps
-    // are as long as the projected problem, 189 -> 146 ms, and 125 -> 115 ms
-    // when the result no longer came by a copy and an event.
+    // residual rule keeps that rare: a step seldom gains a factor of 30.  The
+    // bound on the size is there for a dropped step's price, a product of several
+    // times the projected problem; a cold FP64 solve gains on both sides of it (in
+    // line / ahead, b x b x 2 sites: b = 64 3.95 / 2.83 ms, 256 11.4 / 9.5, 320
+    // 16.9 / 14.6, 448 41.5 / 38.7), a sweep of a settled chain on neither
+    // (chi = 384: 86 / 86 ms), where few solves reach a sixth vector.  Nor do the
+    // precision form's, which end at 1e-5.  A 20-site sweep, chi <= 64: 189 ->
+    // 146 ms, and 125 -> 115 ms when the result no longer came by a copy and an
+    // event.
     RitzLane lane(ctx);
     constexpr int kAheadFrom = 6;
     constexpr long long kAheadElems = 1LL << 17;

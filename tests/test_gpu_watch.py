@@ -156,3 +156,41 @@ def test_chain_calls_report(lib):
     assert lib.lib.nc_test_device_wait(ct.c_uint64(2_000_000_000), ct.c_uint32(0)) == 0
     with pytest.raises(lib.NutcrackerError, match="cluster QR"):
         chain.get_site(7)
+
+
+def test_two_threads_at_once(lib):
+    """Products through residues and panels of both threads in flight together:
+    the bits of a thread alone."""
+    import torch
+    from gpu_util import device_pointers
+
+    args = _product()
+    A, B = device_rand((2, 300, 290), 4), device_rand((2, 290, 200), 5)
+    dims = [ct.c_uint32(v) for v in (300, 290, 200, 2, 2)]
+
+    def work():
+        out = []
+        for _ in range(4):
+            y = heff_dev(lib, *args)
+            oA, oB = torch.empty_like(A), torch.empty_like(B)
+            torch.cuda.current_stream().synchronize()
+            assert lib.lib.nc_gauge_move_dev(ct.c_int(1), *dims, *device_pointers(A, B, oA, oB)) == 0
+            assert lib.lib.nc_synchronize() == 0
+            out.append((y, oA, oB))
+        return out
+
+    ref = work()[0]
+    results = [None, None]
+
+    def run(i):
+        results[i] = work()
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for out in results:
+        assert out is not None
+        for got in out:
+            assert all(torch.equal(x, y) for x, y in zip(got, ref))
