@@ -207,8 +207,11 @@ double residue_scratch_bytes(long long M, long long N, long long K);
 // B(n,k) to p.C[(m % I) + (m / I) * sI + n * sn]: through residues where that
 // pays and holds the operands (scratch from ctx.scratch(); where that cannot be
 // had the product is zgemm(p)).
+// `normwise`: finite operands are multiplied through residues however many of
+// their components are rounded, to 2^-77 of their rows' norms (for factors that
+// are themselves only known to 2^-53 of those).
 void zproduct(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResMatrix& b, int I, long long sI,
-              long long sn);
+              long long sn, bool normwise = false);
 
 // ---- precision form of the site products (mixed.cu) ------------------------
 // Tensor-core operands of one site's H_eff (environments expanded once per

@@ -142,6 +142,7 @@ constexpr Tables make_tables() {
 constexpr Tables kC = make_tables();
 __constant__ Tables kT = make_tables();   // for a modulus known at run time only
 constexpr double kPh = high_part(kP), kPm = mid_part(kP), kPl = low_part(kP);
+constexpr unsigned long long kNormwise = 1ull << 39;   // limit on rounded components that only a non-finite row exceeds
 constexpr int kBadExp = 1 << 30;         // exponent of a row with a non-finite element
 constexpr int kMaxK = 16000;             // |Re|, |Im| sums of K residue products fit in int32
 
@@ -232,7 +233,8 @@ __global__ void __cluster_dims__(PROBE_C, 1, 1) __launch_bounds__(PROBE_T) res_p
     lost = __reduce_add_sync(0xffffffffu, lost);
     if (lane == 0) atomicAdd(cluster.map_shared_rank(&total, 0), lost);
     cluster.sync();
-    if (rank == 0 && threadIdx.x == 0) P.rounded[w2] = total > 2 * ROWS * PROBE_K / 512 ? 1ull << 40 : 0ull;
+    if (rank == 0 && threadIdx.x == 0)
+        P.rounded[w2] = total > 2 * ROWS * PROBE_K / 512 && P.limit[w2] < kNormwise ? 1ull << 40 : 0ull;
 }
 
 // Per (K chunk, row): sum |x|^2 and max(|Re|, |Im|).  K contiguous: one block
@@ -777,7 +779,7 @@ struct ResLayout {
 // C(m,n) = sum_k A(m,k) B(n,k) to C[(m % I) + (m / I) * sI + n * sn] where the
 // operands are held; the gate for the product that runs where they are not.
 ResidueGate residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b, const ResLayout& lay, char* ws, cplx* C,
-                            int I, long long sI, long long sn) {
+                            int I, long long sI, long long sn, bool normwise) {
     ResPair P;
     const ResMatrix* const src[2] = {&a, &b};
     ResidueGate gate;
@@ -796,7 +798,7 @@ ResidueGate residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b
         P.part[w] = reinterpret_cast<double2*>(ws + lay.part[w]);
         P.nb[w] = lay.norm_blocks[w]; P.chunk[w] = lay.chunk[w]; P.nchunk[w] = lay.nchunk[w];
         // random elements leave one component in 2^18 below 2^-24 of a norm (K = 1024); one graded K of a thousand leaves 2^-10
-        P.limit[w] = std::max(4ull, (unsigned long long)m.rows * m.K * 2 >> 15);
+        P.limit[w] = normwise ? kNormwise : std::max(4ull, (unsigned long long)m.rows * m.K * 2 >> 15);
         gate.limit[w] = P.limit[w];
         const long long n = (long long)((P.Kp + CK - 1) / CK) * ((m.rows + CR - 1) / CR);
         nb[w] = (int)n;
@@ -843,7 +845,7 @@ ResidueGate residue_product(Context& ctx, const ResMatrix& a, const ResMatrix& b
 }  // namespace
 
 void zproduct(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResMatrix& b, int I, long long sI,
-              long long sn) {
+              long long sn, bool normwise) {
     NC_ARG(a.K == b.K, "residue product: K");
     ArenaFrame f(ctx.scratch());
     if (!residue_gemm_pays(a.rows, b.rows, a.K)) {
@@ -858,7 +860,7 @@ void zproduct(Context& ctx, const ZGemmParams& p, const ResMatrix& a, const ResM
     profile_launch(ctx, 8.0 * a.rows * (double)b.rows * a.K, 0, [&] {
         ZGemmParams q = p;
         char* ws = ctx.scratch().alloc_n<char>(lay.bytes);
-        q.gate = residue_product(ctx, a, b, lay, ws, p.C, I, sI, sn);
+        q.gate = residue_product(ctx, a, b, lay, ws, p.C, I, sI, sn, normwise);
         zgemm_untimed(q, ctx);
     });
 }
