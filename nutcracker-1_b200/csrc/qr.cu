@@ -548,7 +548,8 @@ cluster_block_qr_kernel(int mp, int nb, int rows_per_cta, cplx* __restrict__ A, 
 // on the FP64 tensor pipe (M = 8 reflectors or columns fits its m8n8k4 shape),
 // with V^H P summed over the CTAs by column slices once per sub-block.  v_c^H v_i for i < c
 // comes out of the column's own sums (they run over all eight columns), so it
-// costs nothing.  B200, one 2048 x 64 block: 212 -> 171 us.
+// costs nothing.  B200, one 2048 x 64 block: 212 -> 174
+// us, 166 in the mean of the sixteen blocks of a 2048 x 1024 QR.
 //
 // The one-block shapes (n <= 64) keep the kernel above: their results stay what
 // they were bit for bit (a chain's edge sites turn rounding into the phase of
@@ -1079,7 +1080,7 @@ void householder_qr(Context& ctx, int m, int n, cplx* A, cplx* Q, cplx* R, bool 
 // so that Q needs no pass per block: once the last block is done,
 // Q(:, :n) = I - V (T V_1^H) (V_1 the top n rows of V) is two large products,
 // through residues where those pay.
-// On a B200 a chi = 1024 move (2048 x 1024) goes from 6.23 to 3.75 ms (with the
+// On a B200 a chi = 1024 move (2048 x 1024) goes from 6.23 to 4.05 ms (with the
 // panels of cluster_subblock_qr_kernel): per block the products between the
 // panels took 130 us on the main stream (partial sums of V^H V and V^H A, T, W2,
 // update), and accumulating Q forwards block by block kept the second stream
