@@ -1319,6 +1319,46 @@ cudaStream_t priority_stream() {
 
 bool q_after(const QrPlan& P) { return residue_gemm_pays(P.n, P.n, P.n) || residue_gemm_pays(P.m, P.n, P.n); }
 
+// Records `once` as the plan's graph.  The result is there already, so a recording
+// that fails costs the graph only, and the next call tries again: the legacy
+// default stream cannot be recorded, and another thread's device-wide
+// synchronisation ends a recording.
+template <typename F>
+void record_qr(Context& ctx, QrPlan& P, F& once) {
+    const uint64_t l0 = ctx.launches;
+    const cudaStream_t home = ctx.stream;
+    const cudaStream_t hp = P.lookahead ? priority_stream() : nullptr;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamBeginCapture(home, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
+        bool whole = false;
+        try {
+            if (hp) {
+                NC_CUDA(cudaEventRecord(P.ev[P.ev.size() - 2], home));
+                NC_CUDA(cudaStreamWaitEvent(hp, P.ev[P.ev.size() - 2], 0));
+                ctx.stream = hp;
+            }
+            once();
+            if (hp) {
+                NC_CUDA(cudaEventRecord(P.ev[P.ev.size() - 1], hp));
+                NC_CUDA(cudaStreamWaitEvent(home, P.ev[P.ev.size() - 1], 0));
+            }
+            whole = true;
+        } catch (...) {
+        }
+        ctx.stream = home;
+        if (cudaStreamEndCapture(home, &graph) != cudaSuccess) graph = nullptr;
+        if (graph && whole && cudaGraphInstantiateWithFlags(&P.exec, graph, cudaGraphInstantiateFlagUseNodePriority) == cudaSuccess) {
+            P.graph = graph;
+            P.kernels = ctx.launches - l0;
+        } else {
+            P.exec = nullptr;
+            if (graph) cudaGraphDestroy(graph);
+        }
+    }
+    cudaGetLastError();
+    ctx.launches = l0;
+}
+
 // Run the QR of plan.X; the first run of a shape executes directly (so the
 // private arena grows to its final size) and then records the graph.
 void qr_run(Context& ctx, QrPlan& P) {
@@ -1339,55 +1379,17 @@ void qr_run(Context& ctx, QrPlan& P) {
         } else
             householder_qr(ctx, P.m, P.n, P.X, P.Q, P.R, P.conjR);
     };
-    if (!P.capture) {
-        try {
-            once();
-        } catch (...) {
-            ctx.ws_override = nullptr;
-            ctx.profile = prof;
-            throw;
-        }
-        ctx.ws_override = nullptr;
-        ctx.profile = prof;
-        return;
-    }
     try {
         once();
-        const uint64_t l0 = ctx.launches;
-        const cudaStream_t home = ctx.stream;
-        const cudaStream_t hp = P.lookahead ? priority_stream() : nullptr;
-        NC_CUDA(cudaStreamBeginCapture(home, cudaStreamCaptureModeRelaxed));
-        try {
-            if (hp) {
-                NC_CUDA(cudaEventRecord(P.ev[P.ev.size() - 2], home));
-                NC_CUDA(cudaStreamWaitEvent(hp, P.ev[P.ev.size() - 2], 0));
-                ctx.stream = hp;
-            }
-            once();
-            if (hp) {
-                NC_CUDA(cudaEventRecord(P.ev[P.ev.size() - 1], hp));
-                ctx.stream = home;
-                NC_CUDA(cudaStreamWaitEvent(home, P.ev[P.ev.size() - 1], 0));
-            }
-        } catch (...) {
-            ctx.stream = home;
-            cudaGraph_t g = nullptr;
-            cudaStreamEndCapture(home, &g);
-            if (g) cudaGraphDestroy(g);
-            throw;
-        }
-        NC_CUDA(cudaStreamEndCapture(home, &P.graph));
-        P.kernels = ctx.launches - l0;
-        ctx.launches = l0;
-        NC_CUDA(cudaGraphInstantiateWithFlags(&P.exec, P.graph, cudaGraphInstantiateFlagUseNodePriority));
     } catch (...) {
         ctx.ws_override = nullptr;
         ctx.profile = prof;
         throw;
     }
+    if (P.capture) record_qr(ctx, P, once);
     ctx.ws_override = nullptr;
     ctx.profile = prof;
-    if (P.lookahead && q_after(P)) qr_form_q(ctx, P.m, P.n, P.V, P.T, P.Q);
+    if (P.lookahead && P.capture && q_after(P)) qr_form_q(ctx, P.m, P.n, P.V, P.T, P.Q);
 }
 }  // namespace
 

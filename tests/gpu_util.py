@@ -43,7 +43,7 @@ def heff_dev(lib, op, L, R, psi, wait=True):
     W = torch.from_numpy(np.ascontiguousarray(op.W.ravel(order="F"))).cuda()
     idx = torch.from_numpy(op.idx.ravel(order="F").astype(np.int32)).cuda()
     y = torch.empty_like(psi)
-    torch.cuda.synchronize()
+    torch.cuda.current_stream().synchronize()   # of this thread's work only: others may be recording graphs
     dims = [ct.c_uint32(v) for v in (bl, br, op.cl, op.cr, d, op.nnz)]
     status = lib.lib.nc_heff_apply_dev(*dims, *device_pointers(idx, W, L, R, psi, y))
     if not wait:
